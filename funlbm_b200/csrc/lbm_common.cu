@@ -128,6 +128,12 @@ Geom make_geom(const lbm_lattice *lat) {
     g.face[i] = lat->face[i];
     for (int k = 0; k < 3; ++k) g.uw[i][k] = lat->face_uw[i][k];
   }
+  const long long wrap[3] = {(g.nx - 1) * g.nyzp, (long long)(g.ny - 1) * g.pz, g.nz - 1};
+  for (int i = 0; i < LBM_NFACES; ++i) {
+    const bool per = g.face[i] == LBM_BC_PERIODICAL;
+    g.foff[i] = per ? (int)((i & 1) == 0 ? wrap[i >> 1] : -wrap[i >> 1]) : 0;
+    g.fwall[i] = per ? 0 : 1;
+  }
   const long long yz = (long long)g.ny * g.nz, xz = (long long)g.nx * g.nz,
                   xy = (long long)g.nx * g.ny;
   g.plane_off[0] = 0;
