@@ -13,8 +13,8 @@ Two representations of the state:
   ``cul_equ``, ``f_stream``, ``update_u_rou``, ``cul_equ2`` act on them one at
   a time (one CUDA kernel each), exactly the reference's call sequence;
 * fused mode -- ``LBMD3.run_step`` advances post-collision populations with
-  one kernel per step; reading an attribute recomputes the reference's state
-  on the device first.
+  one kernel per step; reading an attribute recomputes that part of the
+  reference's state on the device first.
 """
 from __future__ import annotations
 
@@ -168,7 +168,7 @@ class FlowD3(Flow):
         super().__init__(param=param, config=config, device=device)
         self._lat = None
         self._mode = None
-        self._obs_valid = False
+        self._stale = set(self._ALL)
         self._last_force = None
         self._last_fields = ()
         self._tau_t = None
@@ -290,29 +290,54 @@ class FlowD3(Flow):
             self._materialize()
             self._mode = "ref"
 
-    def _materialize(self):
-        if self._obs_valid:
+    # The reference tensors that lag behind the fused state.  Reading an
+    # attribute brings up that tensor alone (u and rho come from one launch):
+    # writing f costs as many bytes again as reading the populations, p and
+    # FOL a pass each, and a program that monitors u and rho asks for none of
+    # them.
+    _ALL = frozenset(("_f", "_u", "_rou", "_p", "_FOL"))
+
+    @property
+    def _obs_valid(self):
+        return not self._stale
+
+    @_obs_valid.setter
+    def _obs_valid(self, valid):
+        self._stale = set() if valid else set(self._ALL)
+
+    def _materialize(self, names=_ALL):
+        need = self._stale.intersection(names)
+        if not need:
             return
         lat = self._lat
         force, fields = self._last_force
-        if self._f is None:        # released while stepping in the fused form
-            self._f = torch.empty((self.q, self.n), device=self.device, dtype=lat.real_dtype)
-        # the kernel writes dense [x][y][z](3) arrays through the raw pointers
-        if not self._rou.is_contiguous():
-            self._rou = self._rou.contiguous()
-        if not self._u.is_contiguous():
-            self._u = self._u.contiguous()
-        lat.observe(force, f=self._f, rho=self._rou, u=self._u)
-        self._p = self._rou / 3.0
-        new_field, new_uniform = fields
-        rdt = lat.real_dtype
-        # the uniform force reaches the kernels as float32
-        g = torch.tensor(new_uniform, device=self.device, dtype=torch.float32).to(rdt)
-        if new_field is not None:
-            self._FOL = new_field.view(self.shape + (3,)) + g
-        else:
-            self._FOL = g.expand(self.shape + (3,)).contiguous()
-        self._obs_valid = True
+        f = rho = u = None
+        if "_f" in need:
+            if self._f is None:        # released while stepping in the fused form
+                self._f = torch.empty((self.q, self.n), device=self.device, dtype=lat.real_dtype)
+            f = self._f
+        if need & {"_u", "_rou"} or ("_p" in need and "_rou" in self._stale):
+            # the kernel writes dense [x][y][z](3) arrays through the raw pointers
+            if not self._rou.is_contiguous():
+                self._rou = self._rou.contiguous()
+            if not self._u.is_contiguous():
+                self._u = self._u.contiguous()
+            rho, u = self._rou, self._u
+            need |= {"_u", "_rou"}
+        if f is not None or u is not None:
+            lat.observe(force, f=f, rho=rho, u=u)
+        if "_p" in need:
+            self._p = self._rou / 3.0
+        if "_FOL" in need:
+            new_field, new_uniform = fields
+            rdt = lat.real_dtype
+            # the uniform force reaches the kernels as float32
+            g = torch.tensor(new_uniform, device=self.device, dtype=torch.float32).to(rdt)
+            if new_field is not None:
+                self._FOL = new_field.view(self.shape + (3,)) + g
+            else:
+                self._FOL = g.expand(self.shape + (3,)).contiguous()
+        self._stale -= need
 
     def enter_fused(self):
         """Start fused stepping from the reference state: the fused kernel
@@ -427,7 +452,7 @@ class FlowD3(Flow):
     # -- attributes ------------------------------------------------------------
     def _get(self, name):
         if self._mode == "fused":
-            self._materialize()
+            self._materialize((name,))
         return getattr(self, name)
 
     def _set(self, name, value):
