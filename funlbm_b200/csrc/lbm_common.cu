@@ -128,12 +128,8 @@ Geom make_geom(const lbm_lattice *lat) {
     g.face[i] = lat->face[i];
     for (int k = 0; k < 3; ++k) g.uw[i][k] = lat->face_uw[i][k];
   }
-  const long long wrap[3] = {(g.nx - 1) * g.nyzp, (long long)(g.ny - 1) * g.pz, g.nz - 1};
-  for (int i = 0; i < LBM_NFACES; ++i) {
-    const bool per = g.face[i] == LBM_BC_PERIODICAL;
-    g.foff[i] = per ? (int)((i & 1) == 0 ? wrap[i >> 1] : -wrap[i >> 1]) : 0;
-    g.fwall[i] = per ? 0 : 1;
-  }
+  for (int i = 0; i < LBM_NFACES; ++i)
+    if (g.face[i] == LBM_BC_WALL_WITH_SPEED) g.moving |= 1u << i;
   const long long yz = (long long)g.ny * g.nz, xz = (long long)g.nx * g.nz,
                   xy = (long long)g.nx * g.ny;
   g.plane_off[0] = 0;
@@ -170,9 +166,24 @@ static void fill_planes_q(const Geom &g, const void *fa, void *fb, int elem, Ste
   using V = VSet<Q>;
   const uintptr_t a = (uintptr_t)fa, b = (uintptr_t)fb;
   auto at = [&](uintptr_t base, long long e) { return base + (uintptr_t)(e * elem); };
+  // element offset of a periodic row's source: the opposite plane
+  const long long wrap[4] = {(g.nx - 1) * g.nyzp, -(g.nx - 1) * g.nyzp, (long long)(g.ny - 1) * g.pz,
+                             -(long long)(g.ny - 1) * g.pz};
+  p.lo = fa;
+  p.hi = (const void *)at(a, (long long)Q * g.np);
   for (int i = 0; i < Q; ++i) {
     const long long plane = (long long)i * g.np, rplane = (long long)V::rev(i) * g.np;
-    p.src[i] = (const void *)at(a, plane - (long long)V::ex(i) * g.nyzp - (long long)V::ey(i) * g.pz);
+    for (int c = 0; c < kRowClasses; ++c) {
+      const int cx = c / 3, cy = c % 3;   // 0 low face, 1 inside, 2 high face
+      int fc = -1;
+      if (V::ex(i) > 0 && cx == 0) fc = 0;
+      if (V::ex(i) < 0 && cx == 2) fc = 1;
+      if (V::ey(i) > 0 && cy == 0) fc = 2;
+      if (V::ey(i) < 0 && cy == 2) fc = 3;
+      p.src[c][i] = (const void *)at(
+          a, fc < 0 ? plane - (long long)V::ex(i) * g.nyzp - (long long)V::ey(i) * g.pz
+                    : g.face[fc] == LBM_BC_PERIODICAL ? plane + wrap[fc] : rplane);
+    }
     p.zlo[i] = nullptr;
     p.zhi[i] = nullptr;
     if (V::ez(i) > 0)

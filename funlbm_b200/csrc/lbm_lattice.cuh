@@ -327,10 +327,7 @@ struct Geom {
   long long np;     // population plane: nx * ny * pz elements
   long long nyzp;   // ny * pz
   int face[LBM_NFACES];
-  // source of a direction entering through a face, relative to the node's
-  // population index: the opposite plane (PERIODICAL) or the node itself, in
-  // the opposite direction (fwall = 1)
-  int foff[LBM_NFACES], fwall[LBM_NFACES];
+  unsigned moving;  // bit fc: face fc is WALL_WITH_SPEED
   float uw[LBM_NFACES][3];
   long long plane_off[LBM_NFACES];  // offsets of the face-density planes
   float tau, inv_tau, cs2, inv_cs2, inv_cs4, force_c;  // force_c = 1 - 1/(2 tau)
@@ -342,6 +339,37 @@ struct Geom {
   double uw_d[LBM_NFACES][3];
 };
 
+// Two float32 values in one register pair (two neighbouring nodes of a row):
+// sm_100's packed add / multiply / fused multiply-add round each half as the
+// scalar instruction does, so a node has the same bits in either form, at
+// half the issue slots.
+struct F2 {
+  float2 v;
+  F2() = default;
+  __device__ __forceinline__ explicit F2(float s) : v(make_float2(s, s)) {}
+  __device__ __forceinline__ F2(float a, float b) : v(make_float2(a, b)) {}
+  __device__ __forceinline__ explicit F2(float2 p) : v(p) {}
+};
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(__fadd2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
+__device__ __forceinline__ F2 operator-(F2 a) { return F2(-a.v.x, -a.v.y); }
+// a - b as a + (-1) b: one rounding, as the subtraction
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
+  return F2(__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v));
+}
+__device__ __forceinline__ F2 &operator+=(F2 &a, F2 b) { return a = a + b; }
+__device__ __forceinline__ F2 &operator-=(F2 &a, F2 b) { return a = a - b; }
+__device__ __forceinline__ F2 fma_rn(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
+__device__ __forceinline__ float recip(float x) { return 1.f / x; }
+__device__ __forceinline__ F2 recip(F2 x) { return F2(1.f / x.v.x, 1.f / x.v.y); }
+// u, zero where the node lies on a boundary plane
+__device__ __forceinline__ float off_face(bool face, float u) { return face ? 0.f : u; }
+struct Face2 {
+  bool a, b;
+};
+__device__ __forceinline__ F2 off_face(Face2 face, F2 u) {
+  return F2(face.a ? 0.f : u.v.x, face.b ? 0.f : u.v.y);
+}
 // Lattice constants in the arithmetic type R of a kernel.
 template <typename R>
 struct Cst;
@@ -360,6 +388,22 @@ struct Cst<double> {
   __device__ __forceinline__ static double inv_cs4(const Geom &g) { return g.inv_cs4_d; }
   __device__ __forceinline__ static double force_c(const Geom &g) { return g.force_c_d; }
   __device__ __forceinline__ static double uw(const Geom &g, int fc, int k) { return g.uw_d[fc][k]; }
+};
+
+template <>
+struct Cst<F2> {
+  __device__ __forceinline__ static F2 inv_cs2(const Geom &g) { return F2(g.inv_cs2); }
+  __device__ __forceinline__ static F2 inv_cs4(const Geom &g) { return F2(g.inv_cs4); }
+  __device__ __forceinline__ static F2 force_c(const Geom &g) { return F2(g.force_c); }
+};
+// type of one node's values in the arithmetic type R
+template <typename R>
+struct OneOf {
+  using type = R;
+};
+template <>
+struct OneOf<F2> {
+  using type = float;
 };
 
 // face-plane index of node (x, y, z) on face `fc`
@@ -389,150 +433,153 @@ __device__ __forceinline__ bool on_any_face(const Geom &g, int x, int y, int z) 
 //   WALL_WITH_SPEED face -> (t, rev(i)) - 2 rho_t w_i (e_i . uw) / cs^2
 // NON_EQUILIBRIUM x faces are handled by the caller (they need moments).
 // ---------------------------------------------------------------------------
-// Source of a direction with component E on one axis: relative offset and
-// bounce-back flag, replaced where it enters through the face of that axis.
-template <int AXIS, int E>
-__device__ __forceinline__ void face_source(const Geom &g, const bool at[LBM_NFACES], int &off,
-                                            int &wall) {
-  if constexpr (E != 0) {
-    constexpr int fc = 2 * AXIS + (E < 0);
-    off = at[fc] ? g.foff[fc] : off;
-    wall = at[fc] ? g.fwall[fc] : wall;
-  }
-}
-
-// Pull of one node with every face rule.  The governing face of direction i
-// is the last one in the order x, y, z whose plane holds the node and through
-// which i enters.  Two phases without a branch between the loads: select each
-// direction's source (foff / fwall: the periodic wrap and the bounce-back flag
-// of each face) and issue all Q loads together, then, only at nodes of a
-// WALL_WITH_SPEED face, subtract its correction (`face_rho`: density of the
-// previous step at this face node).  Chosen over one branch per direction and
-// face, which left each load waiting for the one before it: a warp that
-// touches a face row waited Q memory round trips one after the other
-// (16 steps of a forced 33 x 33 x 65 channel, D3Q19
-// FP32, with the fields read back: 197 -> 111 us; a step of the walled
-// 161 x 65 x 65 sphere case 59 -> 51 us).
-// WORK: return the storage's working value (d for the shifted forms) instead
-// of f; the WALL_WITH_SPEED correction is the same in both (in working
-// units: times 2^kShift).
-template <int Q, int S, bool WORK = false>
-__device__ __forceinline__ void pull_general(const typename Storage<S>::T *__restrict__ fa,
-                                             const Geom &g, int x, int y, int z,
-                                             const typename Storage<S>::R *__restrict__ face_rho,
-                                             typename Storage<S>::R f[Q]) {
-  using V = VSet<Q>;
-  using R = typename Storage<S>::R;
-  const bool at[LBM_NFACES] = {x == 0, x == g.nx - 1, y == 0, y == g.ny - 1, z == 0, z == g.nz - 1};
-  const int sy = g.pz, sx = (int)g.nyzp;
-  const int here = (x * g.ny + y) * sy + z;
-  static_for<Q>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    int off = -(V::ex(i) * sx + V::ey(i) * sy + V::ez(i)), wall = 0;
-    face_source<0, V::ex(i)>(g, at, off, wall);
-    face_source<1, V::ey(i)>(g, at, off, wall);
-    face_source<2, V::ez(i)>(g, at, off, wall);
-    int src = here + off;
-    if (!lbm_in(src >= 0 && src < (int)g.np)) src = here;
-    const unsigned plane = wall ? (unsigned)V::rev(i) : (unsigned)i;
-    const auto *p = fa + ((unsigned long long)plane * (unsigned)g.np + (unsigned)src);
-    if constexpr (WORK)
-      f[i] = Storage<S>::work(p);
-    else
-      f[i] = Storage<S>::load(p, V::template wr<R>(i));   // (w_rev(i) = w_i)
-  });
-  bool moving = false;
-#pragma unroll
-  for (int fc = 0; fc < LBM_NFACES; ++fc)
-    moving = moving || (at[fc] && g.face[fc] == LBM_BC_WALL_WITH_SPEED);
-  if (!moving) return;
-  static_for<Q>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    constexpr int ex = V::ex(i), ey = V::ey(i), ez = V::ez(i);
-    int fc = -1;
-    if constexpr (ex != 0) fc = at[ex < 0] ? (ex < 0) : fc;
-    if constexpr (ey != 0) fc = at[2 + (ey < 0)] ? 2 + (ey < 0) : fc;
-    if constexpr (ez != 0) fc = at[4 + (ez < 0)] ? 4 + (ez < 0) : fc;
-    if (fc >= 0 && g.face[fc] == LBM_BC_WALL_WITH_SPEED) {
-      const R rho_t = face_rho[plane_index(g, fc, x, y, z)];
-      const R eu = (R)ex * Cst<R>::uw(g, fc, 0) + (R)ey * Cst<R>::uw(g, fc, 1) +
-                   (R)ez * Cst<R>::uw(g, fc, 2);
-      const R corr = R(2) * (rho_t * V::template wr<R>(i)) * eu * Cst<R>::inv_cs2(g);
-      f[i] -= WORK ? corr * R(1 << Storage<S>::kShift) : corr;
-    }
-  });
-}
-
 constexpr int kMaxQ = 27;
+
+// Which of a row's faces its nodes lie on (a row: fixed x and y).
+struct RowFaces {
+  bool xl, xh, yl, yh;
+  __device__ __forceinline__ RowFaces(const Geom &g, int x, int y)
+      : xl(x == 0), xh(x == g.nx - 1), yl(y == 0), yh(y == g.ny - 1) {}
+  // row class: 3 (x low, inside, high) x 3 (y)
+  __device__ __forceinline__ int cls() const { return (xl ? 0 : xh ? 6 : 3) + (yl ? 0 : yh ? 2 : 1); }
+  __device__ __forceinline__ bool any() const { return xl || xh || yl || yh; }
+};
+constexpr int kRowClasses = 9, kInnerRow = 4;
+
+// Whether a direction with components EX, EY enters a row through one of its
+// x / y faces.  Its source is then the opposite plane or the node itself, both
+// without a z shift.
+template <int EX, int EY>
+__device__ __forceinline__ bool enters(const RowFaces &r) {
+  bool e = false;
+  if constexpr (EX > 0) e = e || r.xl;
+  if constexpr (EX < 0) e = e || r.xh;
+  if constexpr (EY > 0) e = e || r.yl;
+  if constexpr (EY < 0) e = e || r.yh;
+  return e;
+}
 
 // Per-direction plane pointers of one step, computed on the host
 // (fill_step_planes), so that every population address in the kernels is
 // one 32 x 32 -> 64-bit multiply-add of the node's population index
 // (x ny + y) pz + z onto a parameter:
-//   src[i] + idx   row (x - ex, y - ey) of plane i of fa at the node's z: the
-//                  pull source of an interior row is src[i] + idx - ez;
+//   src[c][i] + idx  pull source of a row of class c at the node's z: inside,
+//                  row (x - ex, y - ey) of plane i, to be read at z - ez;
+//                  where direction i enters through an x / y face (the last
+//                  of them in the order x, y), the opposite plane of i
+//                  (PERIODICAL) or plane rev(i) of the row itself, read at z;
 //   zlo[i] + idx   (ez > 0) source of a node at z = 0 under the bottom face
-//                  rule: PERIODICAL -> (i, x, y, nz - 1), else (rev i, x, y, 0);
+//                  rule, whatever its row: PERIODICAL -> (i, x, y, nz - 1),
+//                  else (rev i, x, y, 0);
 //   zhi[i] + idx   (ez < 0) source of a node at z = nz - 1 under the top face
 //                  rule: PERIODICAL -> (i, x, y, 0), else (rev i, x, y, nz - 1);
 //   dst[i] + idx   plane i of fb.
+// A face row thus runs the same instructions as an inner one.  (One branch
+// per direction and face instead: each load waited for the one before it, and
+// 1.6 % of the rows of a periodic 256^3 lattice took 13 % of the 16-bit
+// step's time.)
 struct StepPlanes {
-  const void *src[kMaxQ];
+  const void *src[kRowClasses][kMaxQ];
   const void *zlo[kMaxQ];
   const void *zhi[kMaxQ];
   void *dst[kMaxQ];
+  const void *lo, *hi;   // the population buffer (bounds-checked build)
 };
 
-// WALL_WITH_SPEED correction of the directions entering through z face FC
-// (4 = bottom, 5 = top) at a node of an interior row, applied after the
-// plain bounce-back pull: the same expression as pull_one's.
-template <int Q, int FC, int SH = 0, typename R>
-__device__ __forceinline__ void zface_wws(const Geom &g, const R *__restrict__ face_rho,
-                                          int x, int y, int z, R f[Q]) {
+// Densities of the previous step at a node of moving walls, one per axis.
+template <typename R>
+struct WallRho {
+  R v[3];
+  __device__ __forceinline__ WallRho(const Geom &g, const R *__restrict__ face_rho,
+                                     const RowFaces &r, int x, int y, int z) {
+    auto at = [&](int fc, bool on) {
+      return on && ((g.moving >> fc) & 1u) ? face_rho[plane_index(g, fc, x, y, z)] : R(0);
+    };
+    v[0] = at(r.xl ? 0 : 1, r.xl || r.xh);
+    v[1] = at(r.yl ? 2 : 3, r.yl || r.yh);
+    v[2] = at(z == 0 ? 4 : 5, z == 0 || z == g.nz - 1);
+  }
+};
+
+// WALL_WITH_SPEED correction of direction I at a node of that face, applied
+// after the bounce-back pull: the amount to subtract from f (WORK units: times
+// 2^SH), 0 where the governing face (the last in the order x, y, z) is not a
+// moving wall.
+template <int Q, int I, int SH, typename R>
+__device__ __forceinline__ R moving_wall(const Geom &g, const WallRho<R> &rho, const RowFaces &r,
+                                         int z) {
   using V = VSet<Q>;
-  const R rho_t = face_rho[plane_index(g, FC, x, y, z)];
-  static_for<Q>([&](auto ic) {
-    constexpr int i = decltype(ic)::value;
-    constexpr int ez = V::ez(i);
-    if constexpr ((FC == 4 && ez > 0) || (FC == 5 && ez < 0)) {
-      const R eu = (R)V::ex(i) * Cst<R>::uw(g, FC, 0) + (R)V::ey(i) * Cst<R>::uw(g, FC, 1) +
-                   (R)ez * Cst<R>::uw(g, FC, 2);
-      constexpr R w = V::template wr<R>(i) * R(1 << SH);   // working units
-      f[i] = f[i] - R(2) * (rho_t * w) * eu * Cst<R>::inv_cs2(g);
-    }
-  });
+  constexpr int ex = V::ex(I), ey = V::ey(I), ez = V::ez(I);
+  int fc = -1;
+  if constexpr (ex > 0) fc = r.xl ? 0 : fc;
+  if constexpr (ex < 0) fc = r.xh ? 1 : fc;
+  if constexpr (ey > 0) fc = r.yl ? 2 : fc;
+  if constexpr (ey < 0) fc = r.yh ? 3 : fc;
+  if constexpr (ez > 0) fc = z == 0 ? 4 : fc;
+  if constexpr (ez < 0) fc = z == g.nz - 1 ? 5 : fc;
+  if (fc < 0 || !((g.moving >> fc) & 1u)) return R(0);
+  const R rho_t = fc < 2 ? rho.v[0] : fc < 4 ? rho.v[1] : rho.v[2];
+  const R eu = (R)ex * Cst<R>::uw(g, fc, 0) + (R)ey * Cst<R>::uw(g, fc, 1) +
+               (R)ez * Cst<R>::uw(g, fc, 2);
+  return R(2) * (rho_t * V::template wr<R>(I)) * eu * Cst<R>::inv_cs2(g) * R(1 << SH);
 }
 
-// Pull of one node of an interior row (x, y not on a face): every source is
-// in row (x - ex, y - ey) except where the z face rule applies, which is
-// chosen by a select on the address (no branch, so all Q loads issue
-// together).  WORK: working values (d for the shifted storages) as the fused
-// step uses them; otherwise f, with the same values and corrections as
-// pull_general.
+// Whether the node lies on a moving wall.
+__device__ __forceinline__ bool on_moving_wall(const Geom &g, const RowFaces &r, int z) {
+  return g.moving != 0 &&
+         (((r.xl ? 1u : 0u) | (r.xh ? 2u : 0u) | (r.yl ? 4u : 0u) | (r.yh ? 8u : 0u) |
+           (z == 0 ? 16u : 0u) | (z == g.nz - 1 ? 32u : 0u)) & g.moving) != 0;
+}
+
+// Pull of one node with the reference's face rules; no branch between the
+// loads, so all Q of them issue together.  WORK: working values (d for the
+// shifted storages) as the fused step uses them; otherwise f.
 template <int Q, int S, bool WORK>
-__device__ __forceinline__ void pull_row_node(const StepPlanes &p, const Geom &g,
-                                              const typename Storage<S>::R *__restrict__ face_rho,
-                                              unsigned idx, int x, int y, int z,
-                                              typename Storage<S>::R f[Q]) {
+__device__ __forceinline__ void pull_node(const StepPlanes &p, const Geom &g,
+                                          const typename Storage<S>::R *__restrict__ face_rho,
+                                          unsigned idx, int x, int y, int z,
+                                          typename Storage<S>::R f[Q]) {
   using St = Storage<S>;
   using T = typename St::T;
   using V = VSet<Q>;
   const bool bottom = z == 0, top = z == g.nz - 1;
-  static_for<Q>([&](auto ic) {
+  const RowFaces r(g, x, y);
+  auto pull = [&](auto ic, const T *ps, bool shifted) {
     constexpr int i = decltype(ic)::value;
     constexpr int ez = V::ez(i);
-    const T *ps = static_cast<const T *>(p.src[i]) + idx;
-    const T *src = ps;
-    if constexpr (ez > 0) src = bottom ? static_cast<const T *>(p.zlo[i]) + idx : ps - 1;
-    if constexpr (ez < 0) src = top ? static_cast<const T *>(p.zhi[i]) + idx : ps + 1;
+    if constexpr (ez != 0) ps = shifted ? ps - ez : ps;
+    if constexpr (ez > 0) ps = bottom ? static_cast<const T *>(p.zlo[i]) + idx : ps;
+    if constexpr (ez < 0) ps = top ? static_cast<const T *>(p.zhi[i]) + idx : ps;
+    if (!lbm_in(ps >= static_cast<const T *>(p.lo) && ps < static_cast<const T *>(p.hi)))
+      ps = static_cast<const T *>(p.lo);
     if constexpr (WORK)
-      f[i] = St::work(src);
+      f[i] = St::work(ps);
     else
-      f[i] = St::load(src, V::template wr<typename St::R>(i));
-  });
-  constexpr int kSh = WORK ? St::kShift : 0;
-  if (bottom && g.face[4] == LBM_BC_WALL_WITH_SPEED) zface_wws<Q, 4, kSh>(g, face_rho, x, y, z, f);
-  if (top && g.face[5] == LBM_BC_WALL_WITH_SPEED) zface_wws<Q, 5, kSh>(g, face_rho, x, y, z, f);
+      f[i] = St::load(ps, V::template wr<typename St::R>(i));   // (w_rev(i) = w_i)
+  };
+  // Two copies of the loads, so that the plane pointers of an inner row are
+  // parameters at fixed places: with one copy indexed by the row's class,
+  // lattices of odd rows ran 2 to 10 % slower (129^3 D3Q15: 52 -> 58 us).
+  if (!r.any()) {
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      pull(ic, static_cast<const T *>(p.src[kInnerRow][i]) + idx, true);
+    });
+  } else {
+    const void *const *src = p.src[r.cls()];
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      pull(ic, static_cast<const T *>(src[i]) + idx, !enters<V::ex(i), V::ey(i)>(r));
+    });
+  }
+  if (on_moving_wall(g, r, z)) {
+    constexpr int kSh = WORK ? St::kShift : 0;
+    const WallRho<typename St::R> rho(g, face_rho, r, x, y, z);
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      if constexpr (i != 0) f[i] -= moving_wall<Q, i, kSh>(g, rho, r, z);
+    });
+  }
 }
 
 // Rolled value (periodic wrap on every axis, no face rule): what the
@@ -559,6 +606,7 @@ __device__ __forceinline__ float pull_rolled(const float *__restrict__ fa, const
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
+
 #define LBM_FMA(a, b, c) ::lbm::fma_rn((a), (b), (c))
 
 // Moments (flow/d3/base.py:116-133): rho = sum f, u = (sum f e + F/2) / rho,
@@ -590,17 +638,24 @@ __device__ __forceinline__ void moments(const R f[Q], R fx, R fy, R fz, bool fac
   uz = face ? R(0) : LBM_FMA(R(0.5), fz, jz) * inv;
 }
 
-// e_i . v with e_i in {-1, 0, 1}^3, folded at compile time
+// e_i . v with e_i in {-1, 0, 1}^3, folded at compile time: the components in
+// the order x, y, z.  Where the first sign is negative the partial sum is
+// kept negated until a positive component turns it (v_y - v_x for
+// -v_x + v_y): the same bits without a negation.
 template <int Q, int I, typename R>
 __device__ __forceinline__ R edot(R vx, R vy, R vz) {
   using V = VSet<Q>;
   R r = R(0);
-  bool first = true;
+  bool first = true, neg = false;
   auto acc = [&](int e, R v) {
     if (e == 0) return;
     if (first) {
-      r = e > 0 ? v : -v;
+      r = v;
+      neg = e < 0;
       first = false;
+    } else if (neg) {
+      r = e > 0 ? v - r : r + v;
+      neg = e < 0;
     } else {
       r = e > 0 ? r + v : r - v;
     }
@@ -608,7 +663,7 @@ __device__ __forceinline__ R edot(R vx, R vy, R vz) {
   acc(V::ex(I), vx);
   acc(V::ey(I), vy);
   acc(V::ez(I), vz);
-  return r;
+  return neg ? -r : r;
 }
 
 // Forcing term of FlowD3.cul_equ2 (flow/d3/base.py:103-114):
@@ -619,6 +674,7 @@ template <int Q, int SH = 0, typename R>
 __device__ __forceinline__ void add_force(R f[Q], const Geom &g, R ux, R uy, R uz, R fx, R fy,
                                           R fz) {
   using V = VSet<Q>;
+  using One = typename OneOf<R>::type;
   const R inv_cs2 = Cst<R>::inv_cs2(g), force_c = Cst<R>::force_c(g);
   const R uF = LBM_FMA(ux, fx, LBM_FMA(uy, fy, uz * fz));
   const R ax = ux * fx, ay = uy * fy, az = uz * fz;
@@ -626,9 +682,9 @@ __device__ __forceinline__ void add_force(R f[Q], const Geom &g, R ux, R uy, R u
   static_for<Q>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
     constexpr int j = V::rev(i);
-    constexpr R cw = V::template wr<R>(i) * R(1 << SH);     // working units
+    constexpr One cw = V::template wr<One>(i) * One(1 << SH);     // working units
     if constexpr (i == 0) {
-      f[0] = LBM_FMA(force_c * cw, base, f[0]);
+      f[0] = LBM_FMA(force_c * R(cw), base, f[0]);
     } else if constexpr (i < j) {
       R t2 = R(0);
       if constexpr (V::ex(i) != 0) t2 += ax;
@@ -636,7 +692,7 @@ __device__ __forceinline__ void add_force(R f[Q], const Geom &g, R ux, R uy, R u
       if constexpr (V::ez(i) != 0) t2 += az;
       const R shared = LBM_FMA(t2, Cst<R>::inv_cs4(g), base);
       const R eF = edot<Q, i>(fx, fy, fz) * inv_cs2;
-      const R c = force_c * cw;
+      const R c = force_c * R(cw);
       f[i] = LBM_FMA(c, shared + eF, f[i]);
       f[j] = LBM_FMA(c, shared - eF, f[j]);
     }
@@ -690,55 +746,72 @@ __device__ __forceinline__ void collide(R f[Q], const Geom &g, R rho, R ux, R uy
 // so the pair (i, rev(i)) gets A +- B with
 //   A = w (drho - rho |u|^2/(2cs^2)) / tau + (w rho t / (2 tau)) t,  B = w rho t / tau.
 // The forcing term (add_force) is additive and applies to d unchanged.
-template <int Q, int SH = 0>
-__device__ __forceinline__ void dev_moments(const float d[Q], float fx, float fy, float fz,
-                                            bool face, float &rho, float &drho, float &ux,
-                                            float &uy, float &uz) {
+// R: float (one node) or F2 (two); FACE: bool or Face2.  FORCED = false: the
+// force is zero and left out.
+template <int Q, int SH, bool FORCED, typename R, typename FACE>
+__device__ __forceinline__ void dev_moments(const R d[Q], R fx, R fy, R fz, FACE face, R &rho,
+                                            R &drho, R &ux, R &uy, R &uz) {
   using V = VSet<Q>;
-  float r = d[0], jx = 0.f, jy = 0.f, jz = 0.f;
+  R r = d[0], jx = R(0.f), jy = R(0.f), jz = R(0.f);
+  bool jx0 = true, jy0 = true, jz0 = true;   // (folded: 0 + t is t)
   static_for<Q>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
     constexpr int j = V::rev(i);
     if constexpr (i != 0 && i < j) {
-      const float s = d[i] + d[j];
-      const float t = d[i] - d[j];
+      const R s = d[i] + d[j];
+      const R t = d[i] - d[j];
       r += s;
-      if constexpr (V::ex(i) > 0) jx += t;
+      if constexpr (V::ex(i) > 0) jx = jx0 ? t : jx + t;
       if constexpr (V::ex(i) < 0) jx -= t;
-      if constexpr (V::ey(i) > 0) jy += t;
+      if constexpr (V::ex(i) != 0) jx0 = false;
+      if constexpr (V::ey(i) > 0) jy = jy0 ? t : jy + t;
       if constexpr (V::ey(i) < 0) jy -= t;
-      if constexpr (V::ez(i) > 0) jz += t;
+      if constexpr (V::ey(i) != 0) jy0 = false;
+      if constexpr (V::ez(i) > 0) jz = jz0 ? t : jz + t;
       if constexpr (V::ez(i) < 0) jz -= t;
+      if constexpr (V::ez(i) != 0) jz0 = false;
     }
   });
   constexpr float kUnscale = 1.f / (float)(1 << SH);      // d = working value / 2^SH
-  drho = r * kUnscale;
-  rho = 1.f + drho;
-  const float inv = 1.f / rho;
-  ux = face ? 0.f : LBM_FMA(0.5f, fx, jx * kUnscale) * inv;
-  uy = face ? 0.f : LBM_FMA(0.5f, fy, jy * kUnscale) * inv;
-  uz = face ? 0.f : LBM_FMA(0.5f, fz, jz * kUnscale) * inv;
+  if constexpr (SH != 0) {
+    drho = r * R(kUnscale);
+    jx = jx * R(kUnscale);
+    jy = jy * R(kUnscale);
+    jz = jz * R(kUnscale);
+  } else {
+    drho = r;
+  }
+  rho = R(1.f) + drho;
+  const R inv = recip(rho);
+  if constexpr (FORCED) {
+    jx = LBM_FMA(R(0.5f), fx, jx);
+    jy = LBM_FMA(R(0.5f), fy, jy);
+    jz = LBM_FMA(R(0.5f), fz, jz);
+  }
+  ux = off_face(face, jx * inv);
+  uy = off_face(face, jy * inv);
+  uz = off_face(face, jz * inv);
 }
 
-template <int Q, int SH = 0>
-__device__ __forceinline__ void collide_dev(float d[Q], const Geom &g, float rho, float drho,
-                                            float ux, float uy, float uz) {
+template <int Q, int SH, typename R>
+__device__ __forceinline__ void collide_dev(R d[Q], const Geom &g, R rho, R drho, R ux, R uy,
+                                            R uz) {
   using V = VSet<Q>;
-  const float u2 = LBM_FMA(ux, ux, LBM_FMA(uy, uy, uz * uz)) * (0.5f * g.inv_cs2);
-  const float vx = ux * g.inv_cs2, vy = uy * g.inv_cs2, vz = uz * g.inv_cs2;
-  const float om = g.inv_tau, keep = 1.f - g.inv_tau;
-  const float orho = om * rho;
-  const float c = om * LBM_FMA(-rho, u2, drho);
+  const R nu2 = LBM_FMA(ux, ux, LBM_FMA(uy, uy, uz * uz)) * R(-0.5f * g.inv_cs2);   // -|u|^2/(2cs^2)
+  const R ic = R(g.inv_cs2), om = R(g.inv_tau), keep = R(1.f - g.inv_tau);
+  const R vx = ux * ic, vy = uy * ic, vz = uz * ic;
+  const R orho = om * rho;
+  const R c = om * LBM_FMA(rho, nu2, drho);
   static_for<Q>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
     constexpr int j = V::rev(i);
     constexpr float w = V::w(i) * (float)(1 << SH);         // working units
     if constexpr (i == 0) {
-      d[0] = LBM_FMA(d[0], keep, w * c);
+      d[0] = LBM_FMA(d[0], keep, R(w) * c);
     } else if constexpr (i < j) {
-      const float t = edot<Q, i>(vx, vy, vz);
-      const float a = LBM_FMA((orho * (0.5f * w)) * t, t, w * c);
-      const float b = (orho * w) * t;
+      const R t = edot<Q, i>(vx, vy, vz);
+      const R a = LBM_FMA((orho * R(0.5f * w)) * t, t, R(w) * c);
+      const R b = (orho * R(w)) * t;
       d[i] = LBM_FMA(d[i], keep, a + b);
       d[j] = LBM_FMA(d[j], keep, a - b);
     }

@@ -29,6 +29,7 @@ struct StepArgs {
   const void *face_rho_in;
   void *face_rho_out;
   void *obs_f, *obs_rho, *obs_u;
+  int obs_pairs;     // observation buffers take aligned stores of two nodes
   unsigned *status;
   StepPlanes p;
 };
@@ -73,49 +74,65 @@ __device__ __forceinline__ ChunkForce chunk_force(const StepArgs &a, unsigned id
   return c;
 }
 
-// finish_node_m also hands the node's end-of-step moments (the second
-// update_u_rou) to the caller.
-template <int Q, bool FORCE, bool DEV, int SH, typename R>
-__device__ __forceinline__ void finish_node_m(const StepArgs &a, R f[Q], unsigned idx, int x,
-                                              int y, int z, bool face, ChunkForce cf,
-                                              unsigned &bad, R &rho_out, R &ux_out, R &uy_out,
-                                              R &uz_out) {
-  using V = VSet<Q>;
-  R fox = a.go[0], foy = a.go[1], foz = a.go[2];
-  R fnx = a.gn[0], fny = a.gn[1], fnz = a.gn[2];
+// Previous / new force at the node: uniform part plus the fields where the
+// node's chunk carries them.
+template <typename R>
+__device__ __forceinline__ void node_force(const StepArgs &a, unsigned idx, ChunkForce cf, R fo[3],
+                                           R fn[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    fo[k] = a.go[k];
+    fn[k] = a.gn[k];
+  }
   if (cf.old_here) {
     const R *fol = static_cast<const R *>(a.fol_old);
-    fox += fol[3ull * idx];
-    foy += fol[3ull * idx + 1];
-    foz += fol[3ull * idx + 2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fo[k] += fol[3ull * idx + k];
   }
   if (cf.new_here) {
     const R *fol = static_cast<const R *>(a.fol_new);
-    fnx += fol[3ull * idx];
-    fny += fol[3ull * idx + 1];
-    fnz += fol[3ull * idx + 2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) fn[k] += fol[3ull * idx + k];
   }
-  R rho, drho = R(0), ux, uy, uz;
-  if constexpr (DEV)
-    dev_moments<Q, SH>(f, fox, foy, foz, face, rho, drho, ux, uy, uz);
-  else
-    moments<Q>(f, fox, foy, foz, face, rho, ux, uy, uz);
+}
+
+// finish_node_m hands the node's end-of-step moments (the second
+// update_u_rou) to the caller; f is left at the end-of-step populations.
+template <int Q, bool FORCE, bool DEV, int SH, typename R>
+__device__ __forceinline__ void finish_node_m(const StepArgs &a, R f[Q], unsigned idx, int x,
+                                              int y, int z, bool face, ChunkForce cf,
+                                              unsigned &bad, R &rho, R &drho, R &ux, R &uy, R &uz) {
+  R fo[3] = {R(0), R(0), R(0)}, fn[3] = {R(0), R(0), R(0)};
+  if constexpr (FORCE) node_force<R>(a, idx, cf, fo, fn);
+  if constexpr (DEV) {
+    dev_moments<Q, SH, FORCE>(f, fo[0], fo[1], fo[2], face, rho, drho, ux, uy, uz);
+  } else {
+    drho = R(0);
+    moments<Q>(f, fo[0], fo[1], fo[2], face, rho, ux, uy, uz);
+  }
   // Where both the previous and this step's force are zero (everywhere
   // outside the spread chunks when there is no uniform force) cul_equ2 adds
   // nothing and the second moment pass repeats the first, so such nodes skip
   // them -- the same rule in every kernel.  (A zero new force alone is not
   // enough: the second pass drops the previous force from u.)
-  if (FORCE && (fnx != R(0) || fny != R(0) || fnz != R(0) || fox != R(0) || foy != R(0) ||
-                foz != R(0))) {
-    add_force<Q, SH>(f, a.g, ux, uy, uz, fnx, fny, fnz);
+  if (FORCE && (fn[0] != R(0) || fn[1] != R(0) || fn[2] != R(0) || fo[0] != R(0) ||
+                fo[1] != R(0) || fo[2] != R(0))) {
+    add_force<Q, SH>(f, a.g, ux, uy, uz, fn[0], fn[1], fn[2]);
     if constexpr (DEV)
-      dev_moments<Q, SH>(f, fnx, fny, fnz, face, rho, drho, ux, uy, uz);
+      dev_moments<Q, SH, true>(f, fn[0], fn[1], fn[2], face, rho, drho, ux, uy, uz);
     else
-      moments<Q>(f, fnx, fny, fnz, face, rho, ux, uy, uz);
+      moments<Q>(f, fn[0], fn[1], fn[2], face, rho, ux, uy, uz);
   }
   bad |= bad_bits(rho, ux, uy, uz);
   if (face && a.face_rho_out != nullptr)
     write_face_rho<Q>(a.g, static_cast<R *>(a.face_rho_out), x, y, z, rho);
+}
+
+// A node's end-of-step state to the observation buffers.
+template <int Q, bool DEV, int SH, typename R>
+__device__ __forceinline__ void observe_node(const StepArgs &a, const R f[Q], unsigned idx, R rho,
+                                             R ux, R uy, R uz) {
+  using V = VSet<Q>;
   if (a.obs_f != nullptr) {
     R *of = static_cast<R *>(a.obs_f);
     static_for<Q>([&](auto ic) {
@@ -131,24 +148,99 @@ __device__ __forceinline__ void finish_node_m(const StepArgs &a, R f[Q], unsigne
     ou[3ull * idx + 1] = uy;
     ou[3ull * idx + 2] = uz;
   }
-  rho_out = rho;
-  ux_out = ux;
-  uy_out = uy;
-  uz_out = uz;
-  if (a.fb != nullptr) {
-    if constexpr (DEV)
-      collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
-    else
-      collide<Q>(f, a.g, rho, ux, uy, uz);
-  }
 }
 
-template <int Q, bool FORCE, bool DEV, int SH, typename R>
+// What a launch does with its nodes: advance them (collide and store) or
+// write their end-of-step state (a kernel of its own, so the step carries
+// none of that code).
+enum class Op { kStep, kObserve };
+
+template <int Q, bool FORCE, bool DEV, int SH, Op OP, typename R>
 __device__ __forceinline__ void finish_node(const StepArgs &a, R f[Q], unsigned idx, int x,
                                             int y, int z, bool face, ChunkForce cf,
                                             unsigned &bad) {
-  R rho, ux, uy, uz;
-  finish_node_m<Q, FORCE, DEV, SH>(a, f, idx, x, y, z, face, cf, bad, rho, ux, uy, uz);
+  R rho, drho, ux, uy, uz;
+  finish_node_m<Q, FORCE, DEV, SH>(a, f, idx, x, y, z, face, cf, bad, rho, drho, ux, uy, uz);
+  if constexpr (OP == Op::kObserve)
+    observe_node<Q, DEV, SH>(a, f, idx, rho, ux, uy, uz);
+  else if constexpr (DEV)
+    collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
+  else
+    collide<Q>(f, a.g, rho, ux, uy, uz);
+}
+
+// finish_node for two neighbouring nodes (z, z + 1) of a row at once, in
+// packed arithmetic: the same operations in the same order, so the same bits.
+// two: the second node exists (the last of a pitched row's odd length has no
+// partner: its lane holds padding and reports nothing).
+template <int Q, bool FORCE, int SH, Op OP>
+__device__ __forceinline__ void finish_pair(const StepArgs &a, F2 f[Q], unsigned idx, int x, int y,
+                                            int z, bool row_face, bool two, ChunkForce c0,
+                                            ChunkForce c1, unsigned &bad) {
+  Face2 face;
+  face.a = row_face || z == 0 || z == a.g.nz - 1;
+  face.b = row_face || z + 1 == a.g.nz - 1;
+  F2 rho, drho, ux, uy, uz;
+  F2 fo[3] = {F2(0.f), F2(0.f), F2(0.f)}, fn[3] = {F2(0.f), F2(0.f), F2(0.f)};
+  if constexpr (FORCE) {
+    float o0[3], n0[3], o1[3], n1[3];
+    node_force<float>(a, idx, c0, o0, n0);
+    node_force<float>(a, two ? idx + 1 : idx, two ? c1 : c0, o1, n1);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      fo[k] = F2(o0[k], o1[k]);
+      fn[k] = F2(n0[k], n1[k]);
+    }
+  }
+  dev_moments<Q, SH, FORCE>(f, fo[0], fo[1], fo[2], face, rho, drho, ux, uy, uz);
+  if constexpr (FORCE) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      any = any || fo[k].v.x != 0.f || fo[k].v.y != 0.f || fn[k].v.x != 0.f || fn[k].v.y != 0.f;
+    if (any) {   // (a node without force next to one that has some is left unchanged by both)
+      add_force<Q, SH>(f, a.g, ux, uy, uz, fn[0], fn[1], fn[2]);
+      dev_moments<Q, SH, true>(f, fn[0], fn[1], fn[2], face, rho, drho, ux, uy, uz);
+    }
+  }
+  bad |= bad_bits(rho.v.x, ux.v.x, uy.v.x, uz.v.x);
+  if (two) bad |= bad_bits(rho.v.y, ux.v.y, uy.v.y, uz.v.y);
+  if (a.face_rho_out != nullptr) {
+    float *fr = static_cast<float *>(a.face_rho_out);
+    if (face.a) write_face_rho<Q>(a.g, fr, x, y, z, rho.v.x);
+    if (face.b && two) write_face_rho<Q>(a.g, fr, x, y, z + 1, rho.v.y);
+  }
+  if constexpr (OP == Op::kStep) {
+    collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
+  } else {
+    if (!two || !a.obs_pairs) {
+      float fa[Q], fb[Q];
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        fa[i] = f[i].v.x;
+        fb[i] = f[i].v.y;
+      });
+      observe_node<Q, true, SH>(a, fa, idx, rho.v.x, ux.v.x, uy.v.x, uz.v.x);
+      if (two) observe_node<Q, true, SH>(a, fb, idx + 1, rho.v.y, ux.v.y, uy.v.y, uz.v.y);
+      return;
+    }
+    if (a.obs_f != nullptr) {
+      float *of = static_cast<float *>(a.obs_f);
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        const F2 v = f[i] * F2(1.f / (float)(1 << SH)) + F2(VSet<Q>::w(i));
+        *reinterpret_cast<float2 *>(of + (long long)i * a.g.n + idx) = v.v;
+      });
+    }
+    if (a.obs_rho != nullptr)
+      *reinterpret_cast<float2 *>(static_cast<float *>(a.obs_rho) + idx) = rho.v;
+    if (a.obs_u != nullptr) {
+      float2 *ou = reinterpret_cast<float2 *>(static_cast<float *>(a.obs_u) + 3ull * idx);
+      ou[0] = make_float2(ux.v.x, uy.v.x);
+      ou[1] = make_float2(uz.v.x, ux.v.y);
+      ou[2] = make_float2(uy.v.y, uz.v.y);
+    }
+  }
 }
 
 __device__ __forceinline__ void report_bad(unsigned *status, unsigned bad) {
@@ -183,7 +275,6 @@ __device__ __forceinline__ void put_padding_vector(const StepArgs &a, unsigned p
   using St = Storage<S>;
   using T = typename St::T;
   constexpr int kWords = NZ * St::kBits / 32;
-  if (a.fb == nullptr) return;
   Words<kWords> zero;
 #pragma unroll
   for (int k = 0; k < kWords; ++k) zero.w[k] = 0u;
@@ -194,12 +285,11 @@ __device__ __forceinline__ void put_padding_vector(const StepArgs &a, unsigned p
 }
 
 // One node per thread, nodes in memory order so that each warp owns one
-// 32-node chunk.  Rows with interior (x, y) pull through pull_row_node;
-// rows on an x / y face take the general face rules.  FORCE adds cul_equ2
+// 32-node chunk.  FORCE adds cul_equ2
 // and the second moment pass; without it both are exact no-ops (the
 // reference adds zeros and recomputes identical moments), so they are
 // skipped.
-template <int Q, int S, bool FORCE>
+template <int Q, int S, bool FORCE, Op OP = Op::kStep>
 __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsigned idx) {
   using St = Storage<S>;
   using T = typename St::T;
@@ -211,17 +301,13 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
   if (!lbm_in(x < a.g.nx && y < a.g.ny && z < a.g.nz && pidx < (unsigned)a.g.np)) return;
   using R = typename St::R;
   const R *face_rho = static_cast<const R *>(a.face_rho_in);
-  const bool row_in = x > 0 && x < a.g.nx - 1 && y > 0 && y < a.g.ny - 1;
   R f[Q];
-  if (row_in)
-    pull_row_node<Q, S, true>(a.p, a.g, face_rho, pidx, x, y, z, f);
-  else
-    pull_general<Q, S, true>(static_cast<const T *>(a.fa), a.g, x, y, z, face_rho, f);
+  pull_node<Q, S, true>(a.p, a.g, face_rho, pidx, x, y, z, f);
   unsigned bad = 0;
-  finish_node<Q, FORCE, St::kDev, St::kShift>(a, f, idx, x, y, z, !row_in || z == 0 || z == a.g.nz - 1, cf,
-                                  bad);
+  finish_node<Q, FORCE, St::kDev, St::kShift, OP>(a, f, idx, x, y, z, on_any_face(a.g, x, y, z), cf,
+                                                  bad);
   report_bad(a.status, bad);
-  if (a.fb != nullptr) {
+  if constexpr (OP == Op::kStep) {
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       St::put(static_cast<T *>(a.p.dst[i]) + pidx, f[i]);
@@ -233,25 +319,38 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
 
 // Register cap of the one-node kernel (resident blocks per SM asked of the
 // compiler, 0 = none).  The one-node kernel runs the rows of odd length (the
-// reference's size + 1 nodes) and is latency-bound there: an ncu capture of
-// the forced D3Q27 FP32 step on 257 x 129 x 129 nodes showed 74 registers,
-// 3 resident blocks of 256 (24 warps / SM) and 7.7 long-scoreboard stalls
-// per issue.  D3Q19 in FP32 and 16-bit storage: 48 registers (5 blocks; the
-// forced 16-bit kernel spills a few words); D3Q27 in FP32 and 16-bit: 64
-// registers (4 blocks), no spills.
+// reference's size + 1 nodes) and is latency-bound there: more resident warps
+// pay until the compiler spills.  Measured on B200, us per step without / with
+// the cap: D3Q19 161 x 65 x 65 fp32 19.0 / 18.5, fp16s 15.1 / 13.3; 177 x 113
+// x 97 fp16s 41.3 / 36.3; D3Q15 129^3 fp32 52.1 / 50.1, fp16s 48.3 / 44.8;
+// D3Q27 257 x 129 x 129 fp32 162 with 4 blocks, 180 with 5; fp16s 120, 124
+// with 5, and 110 uncapped in blocks of 128 threads.
 template <int Q, int S>
 constexpr int scalar_min_blocks() {
   constexpr int bits = Storage<S>::kBits;
   if (bits == 64) return 0;
-  if (Q == 19) return 5;
-  if (Q == 27) return 4;
-  return 0;
+  if (bits == 16) return Q == 27 ? 0 : 5;
+  return Q == 27 ? 4 : 5;
+}
+// Threads per block of the one-node kernel.
+template <int Q, int S>
+__host__ __device__ constexpr int scalar_threads() {
+  return Q == 27 && Storage<S>::kBits == 16 ? 128 : kThreads;
 }
 
 template <int Q, int S, bool FORCE>
-__global__ void __launch_bounds__(kThreads, (scalar_min_blocks<Q, S>())) k_step(const __grid_constant__ StepArgs a) {
+__global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q, S>()))
+    k_step(const __grid_constant__ StepArgs a) {
   chain_enter();
-  step_scalar_body<Q, S, FORCE>(a, blockIdx.x * kThreads + threadIdx.x);
+  step_scalar_body<Q, S, FORCE>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
+}
+
+// The end-of-step state of every node to the observation buffers, nothing
+// stored back: one node per thread (rows that take no pairs, FP64).
+template <int Q, int S, bool FORCE>
+__global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q, S>()))
+    k_observe(const __grid_constant__ StepArgs a) {
+  step_scalar_body<Q, S, FORCE, Op::kObserve>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -289,7 +388,6 @@ template <int Q, int S, bool FORCE>
 __global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__ StepArgs a,
                                                          unsigned long long *out) {
   using St = Storage<S>;
-  using T = typename St::T;
   using R = typename St::R;
   using V = VSet<Q>;
   __shared__ StatAcc sh[kStatsThreads / 32];
@@ -306,17 +404,13 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__
     int x, y, z;
     const ChunkForce cf = chunk_force<FORCE>(a, idx);
     a.dec(idx, x, y, z);
-    const bool row_in = x > 0 && x < a.g.nx - 1 && y > 0 && y < a.g.ny - 1;
     const unsigned pidx = (unsigned)(x * a.g.ny + y) * (unsigned)a.g.pz + (unsigned)z;
     if (!lbm_in(x < a.g.nx && y < a.g.ny && z < a.g.nz && pidx < (unsigned)a.g.np)) continue;
     R f[Q];
-    if (row_in)
-      pull_row_node<Q, S, true>(a.p, a.g, face_rho, pidx, x, y, z, f);
-    else
-      pull_general<Q, S, true>(static_cast<const T *>(a.fa), a.g, x, y, z, face_rho, f);
-    R rho, ux, uy, uz;
-    finish_node_m<Q, FORCE, St::kDev, St::kShift>(a, f, idx, x, y, z, !row_in || z == 0 || z == a.g.nz - 1,
-                                      cf, bad, rho, ux, uy, uz);
+    pull_node<Q, S, true>(a.p, a.g, face_rho, pidx, x, y, z, f);
+    R rho, drho, ux, uy, uz;
+    finish_node_m<Q, FORCE, St::kDev, St::kShift>(a, f, idx, x, y, z, on_any_face(a.g, x, y, z), cf,
+                                                  bad, rho, drho, ux, uy, uz);
     R fmn = R(INFINITY), fmx = -R(INFINITY);
     double fsum = 0.0;
     static_for<Q>([&](auto ic) {
@@ -390,211 +484,229 @@ __global__ void k_stats_finish(unsigned long long *out, double n) {
 }
 
 // ---------------------------------------------------------------------------
-// Vectorised fused step: thread = NZ consecutive nodes of one z-row (nz a
+// Vectorised fused step: thread = NZ consecutive nodes of one z-row (pz a
 // multiple of NZ), populations moved as NZ-element vectors (16 / 8 / 4 byte
-// loads and stores).  For rows whose (x, y) is interior every source of
-// direction i lies in row (x - ex, y - ey): one aligned vector load gives
-// NZ - |ez| of the NZ values, one scalar load the remaining one -- from the
-// neighbouring vector, or at z = 0 / z = nz - 1 from the bottom / top face
-// rule, picked by an address select so that all loads issue together.
-// Rows on an x / y face take the per-node face rules (face_row_nodes).
+// loads and stores), float32 arithmetic packed two nodes to an instruction.
+// What bounds it: HBM for FP32; for 16-bit storage, where a node moves half
+// the bytes, the instructions and the registers per node.  Packing the
+// arithmetic, two branches in place of 2 x 10 address selects and face rows
+// that run the inner rows' code took the 16-bit D3Q19 step from ~610 to ~440
+// instructions per node pair.  Measured at 256^3 (one B200, us per step before
+// -> now, 128 threads): D3Q13 bf16s 199 -> 144, D3Q15 bf16s 220 -> 176, D3Q19
+// bf16s 266 -> 205, fp16s 236 -> 226, D3Q27 fp16s 372 -> 334, bf16s 460 -> 338.
+// Staging rows in shared memory instead (persistent blocks, TMA or cp.async
+// rings, up to three stages) measured slower for every set: 266-350 us for
+// D3Q19 fp16s.
 // ---------------------------------------------------------------------------
-// Whether a vector kernel processes face rows node by node (face_row_nodes)
-// or unrolled with the rest: node by node makes the kernel ~40 % smaller,
-// which measured faster on B200 for the forced kernels and for D3Q13 in
-// 16-bit storage, and slower for the other unforced ones.
-template <int Q, int S, bool FORCE>
-__host__ __device__ constexpr bool compact_face_rows() {
-  return FORCE || (Q == 13 && Storage<S>::kBits == 16);
-}
+// One direction's stored elements of a thread's NZ nodes, still packed: the
+// vector at the thread's own z and the element beyond it that the shifted
+// directions pull.
+template <int S, int NZ>
+struct Pulled {
+  Words<(NZ * Storage<S>::kBits + 31) / 32> w;
+  typename Storage<S>::T extra;
+};
 
-// Nodes of a row on an x / y face (under 1 % of a large lattice), or the
-// last nodes of a pitched row under a WALL_WITH_SPEED top face: one at a
-// time through the general face rules, in a loop that is not unrolled and a
-// function that is not inlined, so a vector kernel carries one copy of this
-// code however many places call it (it is reached from two).  The kernels
-// take their StepArgs as __grid_constant__ parameters, so the reference it
-// receives points at the parameter itself (no per-thread copy).  Same
-// per-node arithmetic.  idx0 / pidx0: dense / population index of node (x, y, z0).
-template <int Q, int S, bool FORCE>
-__device__ __forceinline__ void face_row_nodes(const StepArgs &a, unsigned idx0, unsigned pidx0,
-                                            int count, int pad, int x, int y, int z0) {
-  using St = Storage<S>;
-  using T = typename St::T;
-  using R = typename St::R;
-  const T *fa = static_cast<const T *>(a.fa);
-  const R *face_rho = static_cast<const R *>(a.face_rho_in);
-  unsigned bad = 0;
-#pragma unroll 1
-  for (int k = 0; k < count; ++k) {
-    if (!lbm_in(z0 + k < a.g.nz && pidx0 + k < (unsigned)a.g.np && idx0 + k < (unsigned)a.g.n))
-      continue;
-    R f[Q];
-    pull_general<Q, S, true>(fa, a.g, x, y, z0 + k, face_rho, f);
-    // the nodes may lie in two chunks
-    finish_node<Q, FORCE, St::kDev, St::kShift>(a, f, idx0 + k, x, y, z0 + k, on_any_face(a.g, x, y, z0 + k),
-                                    chunk_force<FORCE>(a, idx0 + k), bad);
-    if (a.fb != nullptr) {
-      static_for<Q>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        St::put(static_cast<T *>(a.p.dst[i]) + pidx0 + k, f[i]);
-      });
-      if (k == count - 1 && pad > 0) put_row_padding<Q, S>(a, pidx0 + count, pad, f);
-    }
+// Element k of a pulled vector as a working value.
+template <int S, int NZ>
+__device__ __forceinline__ float elem(const Pulled<S, NZ> &p, int k) {
+  if constexpr (Storage<S>::kBits == 32) {
+    return __uint_as_float(p.w.w[k]);
+  } else {
+    const float2 v = work2<S>(p.w.w[k >> 1]);
+    return (k & 1) ? v.y : v.x;
   }
-  report_bad(a.status, bad);
 }
 
-// 16-bit storage: the vectors stay packed in registers and are unpacked one
-// node pair at a time, right before that pair is finished and stored (one
-// 32-bit word per direction), so a thread holds 2 x Q floats instead of
-// NZ x Q.  Measured on B200 it is the faster form for 2 nodes per thread
-// (fewer registers, more resident warps); for 4 and 8 the fully unpacked
-// form below keeps more independent work per thread and wins.  Same
-// arithmetic per node as every other shape.
-// ALIGNED = false: the pair starts at any index (rows of odd length), so
-// its elements are loaded and stored one by one and its nodes may lie in two
-// different force chunks.
-template <int Q, int S, bool FORCE, int NZ, bool COMPACT, bool ALIGNED = true, bool PITCH = false>
-__device__ __forceinline__ void step_vec_pairs_at(const StepArgs &a, const unsigned pidx0) {
+// NZ consecutive nodes of one z-row per thread (NZ even), worked through as
+// NZ / 2 pairs in packed arithmetic; idx of node 0 is pidx0 in the population
+// buffers.  The vectors stay packed in registers and a pair is unpacked right
+// before it is finished; each direction leaves in one vector store.
+//   One aligned vector load per direction gives NZ - |ez| of the NZ values,
+// one scalar load the remaining one: from the neighbouring vector, or at
+// z = 0 / z = nz - 1 from the bottom / top face rule.  For 16-bit elements two
+// branches per thread, each over all its directions, instead of an address
+// select per direction: 59 instead of 97 instructions per pair (D3Q19), and
+// the loads of both sides still issue together.  A direction that enters
+// through an x / y face takes its vector unshifted.
+//   ALIGNED = false (16-bit, NZ = 2): the pair starts at any index (dense rows
+// of odd length) and moves element by element.
+//   PITCH: rows may carry padding (pz > nz); the last vector of a row may be
+// partial or hold padding only.  Padding is stored with the vector (see
+// put_row_padding); its lanes report and observe nothing.
+template <int Q, int S, bool FORCE, int NZ, bool PITCH, Op OP = Op::kStep, bool ALIGNED = true>
+__device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned pidx0) {
   using St = Storage<S>;
   using T = typename St::T;
   using V = VSet<Q>;
-  static_assert(St::kBits == 16 && NZ % 2 == 0, "pairs of 16-bit elements");
-  static_assert(ALIGNED || NZ == 2, "unaligned pairs are single pairs");
-  constexpr int kWords = NZ / 2;
+  static_assert(St::kBits <= 32 && NZ % 2 == 0, "pairs of float32 arithmetic");
+  static_assert(ALIGNED || (NZ == 2 && St::kBits == 16), "unaligned pairs are single 16-bit pairs");
+  constexpr int kWords = NZ * St::kBits / 32;
   if (pidx0 >= (unsigned)a.g.np) return;
   int x, y, z0;
   a.pdec(pidx0, x, y, z0);
   if constexpr (PITCH) {
     if (z0 >= a.g.nz) {                      // row padding only
-      put_padding_vector<Q, S, NZ>(a, pidx0);
+      if constexpr (OP == Op::kStep) put_padding_vector<Q, S, NZ>(a, pidx0);
       return;
     }
   }
   const unsigned idx0 = (unsigned)(x * a.g.ny + y) * (unsigned)a.g.nz + (unsigned)z0;
-  // nodes inside the row (fewer than NZ in the last vector of a pitched row:
-  // the other lanes are padding, loaded and stored but not finished)
-  const int nv = PITCH && a.g.nz - z0 < NZ ? a.g.nz - z0 : NZ;
-  if (PITCH && nv < NZ && a.g.face[5] == LBM_BC_WALL_WITH_SPEED) {
-    face_row_nodes<Q, S, FORCE>(a, idx0, pidx0, nv, NZ - nv, x, y, z0);
-    return;
-  }
+  const int nv = PITCH && a.g.nz - z0 < NZ ? a.g.nz - z0 : NZ;    // nodes inside the row
   if (!lbm_in(x < a.g.nx && y < a.g.ny && pidx0 + NZ <= (unsigned)a.g.np &&
               idx0 + nv <= (unsigned)a.g.n))
     return;
-  constexpr bool kCompact = COMPACT;
-  bool row_in = x > 0 && x < a.g.nx - 1 && y > 0 && y < a.g.ny - 1;
-  if constexpr (kCompact) {
-    if (!row_in) {
-      face_row_nodes<Q, S, FORCE>(a, idx0, pidx0, nv, NZ - nv, x, y, z0);
-      return;
-    }
-    row_in = true;
+  // (a thread's nodes may lie in two force chunks: dense rows of any length)
+  const ChunkForce cf0 = chunk_force<FORCE>(a, idx0);
+  ChunkForce cf1 = cf0;
+  if constexpr (FORCE) {
+    if (((idx0 + nv - 1) >> 5) != (idx0 >> 5)) cf1 = chunk_force<FORCE>(a, idx0 + nv - 1);
   }
   const bool bottom = z0 == 0, top = z0 + NZ >= a.g.nz;
-  // lane of the row's last node when it lies inside this vector (else NZ)
-  const int last = nv < NZ ? nv - 1 : NZ;
-  Words<kWords> raw[Q];
-  T extra[Q];
-  if (row_in) {
+  const RowFaces rf(a.g, x, y);
+  const void *const *src = a.p.src[rf.cls()];
+  unsigned bad = 0;
+  Pulled<S, NZ> in[Q];
+  static_for<Q>([&](auto ic) {
+    constexpr int i = decltype(ic)::value;
+    const T *ps = static_cast<const T *>(src[i]) + pidx0;
+    if constexpr (ALIGNED)
+      in[i].w = ld_words<kWords>(ps);
+    else
+      in[i].w.w[0] = (unsigned)bits16(St::raw(ps)) | ((unsigned)bits16(St::raw(ps + 1)) << 16);
+  });
+  if constexpr (St::kBits == 32) {
+    // (select: 0.5 % faster than the branches at 512^3, D3Q19)
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      const T *ps = static_cast<const T *>(src[i]) + pidx0;
+      if constexpr (V::ez(i) > 0)
+        in[i].extra = St::raw(bottom ? static_cast<const T *>(a.p.zlo[i]) + pidx0 : ps - 1);
+      if constexpr (V::ez(i) < 0)
+        in[i].extra =
+            St::raw(top ? static_cast<const T *>(a.p.zhi[i]) + (pidx0 + (nv - 1)) : ps + NZ);
+    });
+  } else {
+    if (bottom) {
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if constexpr (V::ez(i) > 0)
+          in[i].extra = St::raw(static_cast<const T *>(a.p.zlo[i]) + pidx0);
+      });
+    } else {
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if constexpr (V::ez(i) > 0)
+          in[i].extra = St::raw(static_cast<const T *>(src[i]) + pidx0 - 1);
+      });
+    }
+    if (top) {
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if constexpr (V::ez(i) < 0)
+          in[i].extra = St::raw(static_cast<const T *>(a.p.zhi[i]) + (pidx0 + (nv - 1)));
+      });
+    } else {
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        if constexpr (V::ez(i) < 0)
+          in[i].extra = St::raw(static_cast<const T *>(src[i]) + pidx0 + NZ);
+      });
+    }
+  }
+  Words<kWords> out[OP == Op::kStep ? Q : 1];
+#pragma unroll
+  for (int pr = 0; pr < NZ / 2; ++pr) {
+    const int k0 = 2 * pr, k1 = 2 * pr + 1;
+    F2 f[Q];
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       constexpr int ez = V::ez(i);
-      const T *ps = static_cast<const T *>(a.p.src[i]) + pidx0;
-      if constexpr (ALIGNED)
-        raw[i] = ld_words<kWords>(ps);
-      else
-        raw[i].w[0] = (unsigned)bits16(St::raw(ps)) | ((unsigned)bits16(St::raw(ps + 1)) << 16);
-      if constexpr (ez > 0)
-        extra[i] = St::raw(bottom ? static_cast<const T *>(a.p.zlo[i]) + pidx0 : ps - 1);
-      if constexpr (ez < 0)
-        extra[i] = St::raw(top ? static_cast<const T *>(a.p.zhi[i]) + (pidx0 + (nv - 1)) : ps + NZ);
+      const float c0 = elem<S, NZ>(in[i], k0), c1 = elem<S, NZ>(in[i], k1);
+      if constexpr (ez == 0) {
+        f[i] = F2(c0, c1);
+      } else {
+        const float e = St::cvt(in[i].extra);
+        float s0, s1;
+        if constexpr (ez > 0) {
+          s0 = pr == 0 ? e : elem<S, NZ>(in[i], pr == 0 ? 0 : k0 - 1);
+          s1 = c0;
+        } else {
+          s0 = c1;
+          s1 = k1 == NZ - 1 ? e : elem<S, NZ>(in[i], k1 == NZ - 1 ? k1 : k1 + 1);
+        }
+        if constexpr (V::ex(i) != 0 || V::ey(i) != 0) {
+          const bool in_row = enters<V::ex(i), V::ey(i)>(rf);
+          // (at the bottom / top plane the z face's rule governs)
+          s0 = in_row && !(ez > 0 && pr == 0 && bottom) ? c0 : s0;
+          s1 = in_row && !(ez < 0 && k1 == NZ - 1 && top) ? c1 : s1;
+        }
+        if constexpr (PITCH && ez < 0) {
+          // (partial vector: the row's last node is lane nv - 1; the padding
+          // lanes after it keep any value)
+          s0 = top && k0 == nv - 1 ? e : s0;
+          s1 = top && k1 == nv - 1 ? e : s1;
+        }
+        f[i] = F2(s0, s1);
+      }
     });
-  }
-  unsigned bad = 0;
-#pragma unroll
-  for (int pr = 0; pr < kWords; ++pr) {
-    float f0[Q], f1[Q];
-    const int za = z0 + 2 * pr;
-    if (row_in) {
+    if (k0 < nv && (on_moving_wall(a.g, rf, z0 + k0) ||
+                    (k1 < nv && on_moving_wall(a.g, rf, z0 + k1)))) {
+      const float *face_rho = static_cast<const float *>(a.face_rho_in);
+      const int za = z0 + k0, zb = k1 < nv ? z0 + k1 : za;   // (a padding lane repeats its neighbour's)
+      const WallRho<float> rho0(a.g, face_rho, rf, x, y, za), rho1(a.g, face_rho, rf, x, y, zb);
       static_for<Q>([&](auto ic) {
         constexpr int i = decltype(ic)::value;
-        constexpr int ez = V::ez(i);
-        const float2 v = work2<S>(raw[i].w[pr]);
-        if constexpr (ez == 0) {
-          f0[i] = v.x;
-          f1[i] = v.y;
-        } else if constexpr (ez > 0) {
-          f0[i] = pr == 0 ? St::cvt(extra[i]) : work2<S>(raw[i].w[pr > 0 ? pr - 1 : 0]).y;
-          f1[i] = v.x;
-        } else {
-          // (the row's last node pulls the top face's value; a padding lane
-          // after it keeps any value: it is not finished)
-          f0[i] = 2 * pr == last ? St::cvt(extra[i]) : v.y;
-          f1[i] = pr == kWords - 1 || 2 * pr + 1 == last
-                      ? St::cvt(extra[i])
-                      : work2<S>(raw[i].w[pr < kWords - 1 ? pr + 1 : pr]).x;
+        if constexpr (i != 0) {
+          f[i].v.x -= moving_wall<Q, i, St::kShift>(a.g, rho0, rf, za);
+          f[i].v.y -= moving_wall<Q, i, St::kShift>(a.g, rho1, rf, zb);
         }
       });
-      if (pr == 0 && bottom && a.g.face[4] == LBM_BC_WALL_WITH_SPEED)
-        zface_wws<Q, 4, St::kShift>(a.g, static_cast<const float *>(a.face_rho_in), x, y, 0, f0);
-      if (pr == kWords - 1 && top && a.g.face[5] == LBM_BC_WALL_WITH_SPEED)
-        zface_wws<Q, 5, St::kShift>(a.g, static_cast<const float *>(a.face_rho_in), x, y, a.g.nz - 1, f1);
-    } else if constexpr (!kCompact) {
-      const T *fa = static_cast<const T *>(a.fa);
-      const float *face_rho = static_cast<const float *>(a.face_rho_in);
-      // (padding lanes repeat the row's last node; they are not finished)
-      pull_general<Q, S, true>(fa, a.g, x, y, 2 * pr < nv ? za : a.g.nz - 1, face_rho, f0);
-      pull_general<Q, S, true>(fa, a.g, x, y, 2 * pr + 1 < nv ? za + 1 : a.g.nz - 1, face_rho, f1);
     }
-    // (a pair may straddle two force chunks: dense rows of any length)
-    if (2 * pr < nv)
-      finish_node<Q, FORCE, true, St::kShift>(a, f0, idx0 + 2 * pr, x, y, za,
-                                  !row_in || za == 0 || za == a.g.nz - 1,
-                                  chunk_force<FORCE>(a, idx0 + 2 * pr), bad);
-    if (2 * pr + 1 < nv)
-      finish_node<Q, FORCE, true, St::kShift>(a, f1, idx0 + 2 * pr + 1, x, y, za + 1,
-                                  !row_in || za + 1 == a.g.nz - 1,
-                                  chunk_force<FORCE>(a, idx0 + 2 * pr + 1), bad);
-    if (a.fb != nullptr) {
+    if (!PITCH || k0 < nv) {
+      const bool s0 = ((idx0 + k0) >> 5) == (idx0 >> 5), s1 = ((idx0 + k1) >> 5) == (idx0 >> 5);
+      finish_pair<Q, FORCE, St::kShift, OP>(a, f, idx0 + k0, x, y, z0 + k0, rf.any(),
+                                            !PITCH || k1 < nv, s0 ? cf0 : cf1, s1 ? cf0 : cf1,
+                                            bad);
+    }
+    if constexpr (OP == Op::kStep) {
       static_for<Q>([&](auto ic) {
         constexpr int i = decltype(ic)::value;
-        T *dst = static_cast<T *>(a.p.dst[i]) + pidx0 + 2 * pr;
-        const unsigned word = put2<S>(f0[i], f1[i]);
-        if constexpr (ALIGNED) {
-          st_words(dst, Words<1>{{word}});
+        if constexpr (St::kBits == 32) {
+          out[i].w[k0] = __float_as_uint(f[i].v.x);
+          out[i].w[k1] = __float_as_uint(f[i].v.y);
         } else {
-          reinterpret_cast<unsigned short *>(dst)[0] = (unsigned short)(word & 0xffffu);
-          reinterpret_cast<unsigned short *>(dst)[1] = (unsigned short)(word >> 16);
+          out[i].w[pr] = put2<S>(f[i].v.x, f[i].v.y);
         }
       });
     }
   }
   report_bad(a.status, bad);
+  if constexpr (OP == Op::kStep) {
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      T *dst = static_cast<T *>(a.p.dst[i]) + pidx0;
+      if constexpr (ALIGNED) {
+        st_words(dst, out[i]);
+      } else {
+        reinterpret_cast<unsigned short *>(dst)[0] = (unsigned short)(out[i].w[0] & 0xffffu);
+        reinterpret_cast<unsigned short *>(dst)[1] = (unsigned short)(out[i].w[0] >> 16);
+      }
+    });
+  }
 }
 
-template <int Q, int S, bool FORCE, int NZ, bool COMPACT, bool PITCH>
-__device__ __forceinline__ void step_vec_pairs(const StepArgs &a, const unsigned t) {
-  step_vec_pairs_at<Q, S, FORCE, NZ, COMPACT, true, PITCH>(a, t * NZ);
-}
-
-
-// PITCH: rows may carry padding (pz > nz) -- the kernel then handles a
-// partial last vector per row and writes the padding; lattices without
-// padding run the variant that has none of that code.
-template <int Q, int S, bool FORCE, int NZ, bool PITCH,
-          bool COMPACT = compact_face_rows<Q, S, FORCE>()>
-__device__ __forceinline__ void step_vec_body(const StepArgs &a, const unsigned t) {
+// Vectorised step of FP64 rows (pz = nz or padded): thread = NZ consecutive
+// nodes, pulled and finished node by node in double arithmetic, stored as
+// vectors.
+template <int Q, int S, bool FORCE, int NZ, bool PITCH>
+__device__ __forceinline__ void step_vec64_body(const StepArgs &a, const unsigned t) {
   using St = Storage<S>;
   using T = typename St::T;
   using V = VSet<Q>;
-  if constexpr (St::kBits == 16 && NZ == 2) {
-    step_vec_pairs<Q, S, FORCE, NZ, COMPACT, PITCH>(a, t);
-    return;
-  }
   using R = typename St::R;
-  constexpr int kWords = NZ * St::kBits / 32;
+  static_assert(St::kBits == 64, "float64 rows");
+  constexpr int kWords = 2 * NZ;
   const unsigned pidx0 = t * NZ;
   if (pidx0 >= (unsigned)a.g.np) return;
   int x, y, z0;
@@ -606,126 +718,62 @@ __device__ __forceinline__ void step_vec_body(const StepArgs &a, const unsigned 
     }
   }
   const unsigned idx0 = (unsigned)(x * a.g.ny + y) * (unsigned)a.g.nz + (unsigned)z0;
-  // Nodes of this vector inside the row: fewer than NZ in the last vector of
-  // a pitched row, whose other lanes are row padding -- loaded and stored
-  // with the vector (never a pull source, never observed) but not finished.
   const int nv = PITCH && a.g.nz - z0 < NZ ? a.g.nz - z0 : NZ;
-  if (PITCH && nv < NZ && a.g.face[5] == LBM_BC_WALL_WITH_SPEED) {
-    face_row_nodes<Q, S, FORCE>(a, idx0, pidx0, nv, NZ - nv, x, y, z0);
-    return;
-  }
   if (!lbm_in(x < a.g.nx && y < a.g.ny && pidx0 + NZ <= (unsigned)a.g.np &&
               idx0 + nv <= (unsigned)a.g.n))
     return;
-  constexpr bool kCompact = COMPACT;
-  bool row_in = x > 0 && x < a.g.nx - 1 && y > 0 && y < a.g.ny - 1;
-  if constexpr (kCompact) {
-    if (!row_in) {
-      face_row_nodes<Q, S, FORCE>(a, idx0, pidx0, nv, NZ - nv, x, y, z0);
-      return;
-    }
-    row_in = true;
-  }
   const R *face_rho = static_cast<const R *>(a.face_rho_in);
   R f[NZ][Q];
-  if (row_in) {
-    // top: the row's last node is in this vector (lane nv - 1)
-    const bool bottom = z0 == 0, top = z0 + NZ >= a.g.nz;
-    static_for<Q>([&](auto ic) {
-      constexpr int i = decltype(ic)::value;
-      constexpr int ez = V::ez(i);
-      const T *ps = static_cast<const T *>(a.p.src[i]) + pidx0;
-      const Words<kWords> raw = ld_words<kWords>(ps);
-      R v[NZ];
-      if constexpr (St::kBits == 32) {
 #pragma unroll
-        for (int k = 0; k < NZ; ++k) v[k] = __uint_as_float(raw.w[k]);
-      } else if constexpr (St::kBits == 64) {
-#pragma unroll
-        for (int k = 0; k < NZ; ++k) v[k] = __hiloint2double((int)raw.w[2 * k + 1], (int)raw.w[2 * k]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < NZ / 2; ++k) {
-          const float2 p2 = work2<S>(raw.w[k]);
-          v[2 * k] = p2.x;
-          v[2 * k + 1] = p2.y;
-        }
-      }
-      if constexpr (ez == 0) {
-#pragma unroll
-        for (int k = 0; k < NZ; ++k) f[k][i] = v[k];
-      } else if constexpr (ez > 0) {
-#pragma unroll
-        for (int k = 1; k < NZ; ++k) f[k][i] = v[k - 1];
-        f[0][i] = St::work(bottom ? static_cast<const T *>(a.p.zlo[i]) + pidx0 : ps - 1);
-      } else {
-        // the row's last node (lane nv - 1) pulls the top face's value; in a
-        // partial vector the padding lanes after it take any value (a
-        // select per lane, not a store at a computed lane, which would put
-        // f in local memory)
-        const R e = St::work(top ? static_cast<const T *>(a.p.zhi[i]) + (pidx0 + (nv - 1))
-                                 : ps + NZ);
-#pragma unroll
-        for (int k = 0; k < NZ - 1; ++k) f[k][i] = k == nv - 1 ? e : v[k + 1];
-        f[NZ - 1][i] = e;
-      }
-    });
-    if (bottom && a.g.face[4] == LBM_BC_WALL_WITH_SPEED)
-      zface_wws<Q, 4, St::kShift>(a.g, face_rho, x, y, 0, f[0]);
-    if (top && a.g.face[5] == LBM_BC_WALL_WITH_SPEED)
-      zface_wws<Q, 5, St::kShift>(a.g, face_rho, x, y, a.g.nz - 1, f[NZ - 1]);
-  } else if constexpr (!kCompact) {
-    const T *fa = static_cast<const T *>(a.fa);
-    // (padding lanes repeat the row's last node; they are not finished)
-#pragma unroll
-    for (int k = 0; k < NZ; ++k)
-      pull_general<Q, S, true>(fa, a.g, x, y, k < nv ? z0 + k : a.g.nz - 1, face_rho, f[k]);
+  for (int k = 0; k < NZ; ++k) {
+    const int kk = k < nv ? k : nv - 1;   // (padding lanes repeat the row's last node)
+    pull_node<Q, S, true>(a.p, a.g, face_rho, pidx0 + kk, x, y, z0 + kk, f[k]);
   }
-
   unsigned bad = 0;
 #pragma unroll
   for (int k = 0; k < NZ; ++k) {
     const int z = z0 + k;
-    // (a thread's nodes may straddle two force chunks: dense rows of any length)
     if (k < nv)
-      finish_node<Q, FORCE, St::kDev, St::kShift>(a, f[k], idx0 + k, x, y, z,
-                                      !row_in || z == 0 || z == a.g.nz - 1,
-                                      chunk_force<FORCE>(a, idx0 + k), bad);
+      finish_node<Q, FORCE, St::kDev, St::kShift, Op::kStep>(
+          a, f[k], idx0 + k, x, y, z, on_any_face(a.g, x, y, z),
+          chunk_force<FORCE>(a, idx0 + k), bad);
   }
   report_bad(a.status, bad);
-  if (a.fb == nullptr) return;
   static_for<Q>([&](auto ic) {
     constexpr int i = decltype(ic)::value;
     Words<kWords> raw;
-    if constexpr (St::kBits == 32) {
 #pragma unroll
-      for (int k = 0; k < NZ; ++k) raw.w[k] = __float_as_uint(f[k][i]);
-    } else if constexpr (St::kBits == 64) {
-#pragma unroll
-      for (int k = 0; k < NZ; ++k) {
-        raw.w[2 * k] = (unsigned)__double2loint(f[k][i]);
-        raw.w[2 * k + 1] = (unsigned)__double2hiint(f[k][i]);
-      }
-    } else {
-#pragma unroll
-      for (int k = 0; k < NZ / 2; ++k) raw.w[k] = put2<S>(f[2 * k][i], f[2 * k + 1][i]);
+    for (int k = 0; k < NZ; ++k) {
+      raw.w[2 * k] = (unsigned)__double2loint(f[k][i]);
+      raw.w[2 * k + 1] = (unsigned)__double2hiint(f[k][i]);
     }
     st_words(static_cast<T *>(a.p.dst[i]) + pidx0, raw);
   });
+}
+
+// PITCH: rows may carry padding (pz > nz); lattices without padding run the
+// variant that has none of that code.
+template <int Q, int S, bool FORCE, int NZ, bool PITCH>
+__device__ __forceinline__ void step_vec_body(const StepArgs &a, const unsigned t) {
+  if constexpr (Storage<S>::kBits == 64)
+    step_vec64_body<Q, S, FORCE, NZ, PITCH>(a, t);
+  else
+    step_pairs_at<Q, S, FORCE, NZ, PITCH>(a, t * NZ);
 }
 
 // Register cap of the vectorised step for 16-bit storage, as resident blocks
 // per SM asked of the compiler (0 = no cap).  A 16-bit population costs a
 // whole float register once unpacked, so the 16-bit kernels hold too few
 // bytes in flight per SM to cover HBM latency unless enough warps are
-// resident; these caps (measured on B200 at 512^3 and on lattices with
-// particles; none of them spills) trade register slack for resident warps.
-// FP32 runs uncapped.
+// resident (measured on B200 at 256^3, unforced, 128 threads, fraction of the
+// copy peak without / with the cap: D3Q13 4 nodes 0.915 / 0.927, D3Q15 bf16s
+// 4 nodes - / 0.873, D3Q19 4 nodes 0.687 / 0.859, D3Q27 2 nodes 0.821 /
+// 0.828).  FP32 runs uncapped.
 template <int Q, int S, int NZ, bool FORCE>
 constexpr int vec_reg_cap() {
   if (Storage<S>::kBits != 16) return 0;
-  if (NZ == 2 && FORCE) return Q == 19 ? 72 : Q == 27 ? 96 : 0;
-  if (NZ == 4) return Q == 15 || Q == 19 ? 128 : 0;
+  if (NZ == 2) return Q == 27 ? 96 : FORCE && Q == 19 ? 80 : 0;
+  if (NZ == 4) return Q == 13 ? 96 : Q == 15 || Q == 19 ? 128 : 0;
   return 0;
 }
 template <int Q, int S, int NZ, int TB, bool FORCE>
@@ -738,6 +786,12 @@ __global__ void __launch_bounds__(TB, (vec_min_blocks<Q, S, NZ, TB, FORCE>()))
     k_step_vec(const __grid_constant__ StepArgs a) {
   chain_enter();
   step_vec_body<Q, S, FORCE, NZ, PITCH>(a, blockIdx.x * TB + threadIdx.x);
+}
+
+// The end-of-step state to the observation buffers, two nodes per thread.
+template <int Q, int S, bool FORCE, bool PITCH>
+__global__ void __launch_bounds__(128) k_observe_vec(const __grid_constant__ StepArgs a) {
+  step_pairs_at<Q, S, FORCE, 2, PITCH, Op::kObserve>(a, 2u * (blockIdx.x * 128u + threadIdx.x));
 }
 
 // Rows of odd length in 16-bit storage: thread k of a row takes the node pair
@@ -756,7 +810,7 @@ __global__ void __launch_bounds__(TB, (vec_min_blocks<Q, S, 2, TB, FORCE>()))
   const unsigned z = 2u * (t - row * per_row.d);
   const unsigned idx = row * (unsigned)a.g.nz + z;
   if (z + 1u < (unsigned)a.g.nz)
-    step_vec_pairs_at<Q, S, FORCE, 2, compact_face_rows<Q, S, FORCE>(), false>(a, idx);
+    step_pairs_at<Q, S, FORCE, 2, false, Op::kStep, false>(a, idx);
   else
     step_scalar_body<Q, S, FORCE>(a, idx);
 }
@@ -957,29 +1011,34 @@ __global__ void __launch_bounds__(kTmaThreads) k_step_tma(const __grid_constant_
                                 : sm_elem<S>(rp + z + 2);
           }
         });
-        if (z == 0 && a.g.face[4] == LBM_BC_WALL_WITH_SPEED)
-          zface_wws<Q, 4, St::kShift>(a.g, face_rho, x, y, 0, f0);
-        if (z + 2 == nz && a.g.face[5] == LBM_BC_WALL_WITH_SPEED)
-          zface_wws<Q, 5, St::kShift>(a.g, face_rho, x, y, nz - 1, f1);
+        if (a.g.moving != 0 && (z == 0 || z + 2 == nz)) {
+          const RowFaces rf(a.g, x, y);
+          const WallRho<float> rho0(a.g, face_rho, rf, x, y, z), rho1(a.g, face_rho, rf, x, y, z + 1);
+          static_for<Q>([&](auto ic) {
+            constexpr int i = decltype(ic)::value;
+            if constexpr (i != 0) {
+              f0[i] -= moving_wall<Q, i, St::kShift>(a.g, rho0, rf, z);
+              f1[i] -= moving_wall<Q, i, St::kShift>(a.g, rho1, rf, z + 1);
+            }
+          });
+        }
       } else {
-        pull_general<Q, S, true>(fa, a.g, x, y, z, face_rho, f0);
-        pull_general<Q, S, true>(fa, a.g, x, y, z + 1, face_rho, f1);
+        pull_node<Q, S, true>(a.p, a.g, face_rho, idx, x, y, z, f0);
+        pull_node<Q, S, true>(a.p, a.g, face_rho, idx + 1, x, y, z + 1, f1);
       }
       unsigned bad = 0;
-      finish_node<Q, FORCE, St::kDev, St::kShift>(a, f0, idx, x, y, z, !row_in || z == 0, cf, bad);
-      finish_node<Q, FORCE, St::kDev, St::kShift>(a, f1, idx + 1, x, y, z + 1, !row_in || z + 1 == nz - 1, cf,
-                                      bad);
+      finish_node<Q, FORCE, St::kDev, St::kShift, Op::kStep>(a, f0, idx, x, y, z, !row_in || z == 0, cf, bad);
+      finish_node<Q, FORCE, St::kDev, St::kShift, Op::kStep>(a, f1, idx + 1, x, y, z + 1,
+                                                             !row_in || z + 1 == nz - 1, cf, bad);
       report_bad(a.status, bad);
-      if (a.fb != nullptr) {
-        static_for<Q>([&](auto ic) {
-          constexpr int i = decltype(ic)::value;
-          T *dst = static_cast<T *>(a.p.dst[i]) + idx;
-          if constexpr (St::kBits == 32)
-            *reinterpret_cast<float2 *>(dst) = make_float2(f0[i], f1[i]);
-          else
-            *reinterpret_cast<unsigned *>(dst) = put2<S>(f0[i], f1[i]);
-        });
-      }
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        T *dst = static_cast<T *>(a.p.dst[i]) + idx;
+        if constexpr (St::kBits == 32)
+          *reinterpret_cast<float2 *>(dst) = make_float2(f0[i], f1[i]);
+        else
+          *reinterpret_cast<unsigned *>(dst) = put2<S>(f0[i], f1[i]);
+      });
     }
     __syncthreads();
     if (tid == 0) {
@@ -1136,22 +1195,62 @@ struct StepLauncher {
     else
       force ? go_odd_f<true, 128>(a, s) : go_odd_f<false, 128>(a, s);
   }
+  // Observation launch: two nodes per thread where the rows allow pairs.
+  static int go_observe(StepArgs a, bool force, int nodes, cudaStream_t s) {
+    constexpr int bits = Storage<S>::kBits;
+    if (nodes == LBM_STEP_ROWS) {   // (a lattice that cannot be row-staged is refused here too)
+      TmaPlan p;
+      int ctas;
+      size_t smem;
+      unsigned grid;
+      if (bits == 64 || !tma_plan(a.g, Q, bits, a.fa, p, ctas, smem, grid)) return go_tma(a, force, s);
+    }
+    const uintptr_t at = (uintptr_t)a.obs_f | (uintptr_t)a.obs_rho | (uintptr_t)a.obs_u;
+    a.obs_pairs = a.g.n % 2 == 0 && a.g.nz % 2 == 0 && at % 8 == 0;
+    if constexpr (bits != 64) {
+      if (nodes != 1 && step_shape_ok(2, a.g.pz, bits)) {
+        const unsigned nb = blocks_for(a.g.np / 2, 128);
+        const bool pitch = a.g.pz != a.g.nz;
+        if (force)
+          pitch ? launch_chained(k_observe_vec<Q, S, true, true>, nb, 128, 0, s, a)
+                : launch_chained(k_observe_vec<Q, S, true, false>, nb, 128, 0, s, a);
+        else
+          pitch ? launch_chained(k_observe_vec<Q, S, false, true>, nb, 128, 0, s, a)
+                : launch_chained(k_observe_vec<Q, S, false, false>, nb, 128, 0, s, a);
+        return LBM_OK;
+      }
+    }
+    constexpr int tb = scalar_threads<Q, S>();
+    const unsigned nb = blocks_for(a.g.n, tb);
+    if (force)
+      launch_chained(k_observe<Q, S, true>, nb, tb, 0, s, a);
+    else
+      launch_chained(k_observe<Q, S, false>, nb, tb, 0, s, a);
+    return LBM_OK;
+  }
   static int go(const StepArgs &a, bool force, int nodes, int threads, cudaStream_t s) {
     constexpr int bits = Storage<S>::kBits;
+    if (a.fb == nullptr) return go_observe(a, force, nodes, s);
+    if (a.obs_f != nullptr || a.obs_rho != nullptr || a.obs_u != nullptr) {
+      StepArgs o = a;   // (the step below reports the status and the face densities)
+      o.status = nullptr;
+      o.face_rho_out = nullptr;
+      const int rc = go_observe(o, force, nodes, s);
+      if (rc) return rc;
+    }
     if (nodes == LBM_STEP_ROWS) return go_tma(a, force, s);
     const bool odd_pairs = bits == 16 && a.g.pz % 2 == 1 && a.g.nz >= 3;
     if (nodes == 0) {
-      // Measured on B200 at 512^3: node pairs with 128-thread blocks are the
-      // fastest shape wherever rows allow them (D3Q19 FP32 3027 us, one node
-      // per thread 3045 us; 3035 against 3132 us over seconds under the
-      // power cap, where the pair kernel holds 1935 MHz and the other 1845),
-      // except unforced D3Q13 / D3Q19 in 16-bit storage, where 4 nodes per
-      // thread are (D3Q19 fp16s 1818 against 1881 us, bf16s 2075 against
-      // 2325; D3Q13 fp16s 1594 against 1768).  Rows of odd length without
-      // pitch take one node per thread (on the walled 161x65x65 and
-      // 257x129x129 lattices also faster than pitched pairs); the odd-row
-      // pair kernel is a tuner candidate only.
-      const int want = (bits == 16 && (Q == 13 || Q == 19) && !force) ? 4 : 2;
+      // Measured on B200, blocks of 128 threads, fraction of the copy peak for
+      // 2 / 4 nodes per thread (256^3 unless said): FP32 D3Q19 1.02 / 1.00
+      // (512^3 3007 us a step; one node per thread is 1 % slower); 16-bit
+      // D3Q13 0.83 / 0.93; D3Q15 fp16s 0.83 / 0.77, bf16s 0.82 / 0.87; D3Q19
+      // fp16s 0.87 / 0.86 (512^3 0.88 / 0.89), bf16s 0.87 / 0.95; D3Q27 fp16s
+      // 0.83 / 0.82.  Forced kernels keep pairs (4 nodes spill).  Rows of odd
+      // length without pitch take one node per thread; the odd-row pair kernel
+      // is a tuner candidate only.
+      constexpr bool four = bits == 16 && (Q == 13 || Q == 19 || (Q == 15 && S == LBM_STORAGE_BF16S));
+      const int want = four && !force ? 4 : 2;
       nodes = step_shape_ok(want, a.g.pz, bits) ? want : step_shape_ok(2, a.g.pz, bits) ? 2 : 1;
       threads = threads ? threads : 128;
     }
@@ -1175,11 +1274,12 @@ struct StepLauncher {
         return LBM_OK;
       }
     }
-    const unsigned nb = blocks_for(a.g.n, kThreads);
+    constexpr int tb = scalar_threads<Q, S>();
+    const unsigned nb = blocks_for(a.g.n, tb);
     if (force)
-      launch_chained(k_step<Q, S, true>, nb, kThreads, 0, s, a);
+      launch_chained(k_step<Q, S, true>, nb, tb, 0, s, a);
     else
-      launch_chained(k_step<Q, S, false>, nb, kThreads, 0, s, a);
+      launch_chained(k_step<Q, S, false>, nb, tb, 0, s, a);
     return LBM_OK;
   }
 };
