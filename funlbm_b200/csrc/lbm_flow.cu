@@ -61,8 +61,10 @@ __global__ void __launch_bounds__(kThreads)
 // ---------------------------------------------------------------------------
 template <int Q>
 __global__ void __launch_bounds__(kThreads)
-    k_collide(const Geom g, float *f, const float *rho, const float *u, float *feq) {
+    k_collide(const Geom g, float *f, const float *rho, const float *u, float *feq, float *rmax) {
+  chain_enter();
   const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
+  if (rmax != nullptr && idx == 0) *rmax = 0.f;   // (for the moments after the stream)
   if (idx >= (unsigned)g.n) return;
   const float r = rho[idx], ux = u[3ull * idx], uy = u[3ull * idx + 1], uz = u[3ull * idx + 2];
   float fl[Q];
@@ -84,77 +86,77 @@ __global__ void __launch_bounds__(kThreads)
   });
 }
 
-// f_stream + f_stream_bound_* with every face code, NON_EQUILIBRIUM included.
+// f_stream + f_stream_bound_* of one node with every face code: the sources
+// of the step's pull (planes of the dense float32 arrays, no working-value
+// conversion), the moving walls' correction with the node's own density, and
+// at NON_EQUILIBRIUM x faces, for the directions that no y / z face governs,
+// feq + (rolled f - feq) of the neighbouring plane.
 template <int Q>
-__global__ void __launch_bounds__(kThreads) k_stream(const Geom g, const NodeDecomp dec,
-                                                     const float *fin, float *fout,
-                                                     const float *rho, const float *feq) {
+__device__ __forceinline__ void stream_node(const StepPlanes &p, const Geom &g, const float *fin,
+                                            const float *rho, const float *feq, unsigned idx, int x,
+                                            int y, int z, float f[Q]) {
   using V = VSet<Q>;
+  const RowFaces r(g, x, y);
+  pull_sources<Q, LBM_STORAGE_FP32, true>(p, g, r, idx, z, f);
+  if (on_moving_wall(g, r, z)) {
+    const WallRho<float> wr(rho[idx]);
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      if constexpr (i != 0) f[i] -= moving_wall<Q, i, 0>(g, wr, r, z);
+    });
+  }
+  if ((r.xl && g.face[0] == LBM_BC_NON_EQUILIBRIUM) ||
+      (r.xh && g.face[1] == LBM_BC_NON_EQUILIBRIUM)) {
+    const int nbx = r.xl ? 1 : g.nx - 2;
+    const long long nb = ((long long)nbx * g.ny + y) * g.nz + z;
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      constexpr int ey = V::ey(i), ez = V::ez(i);
+      bool other = false;
+      if constexpr (ey != 0) other = other || (ey > 0 ? r.yl : r.yh);
+      if constexpr (ez != 0) other = other || (ez > 0 ? z == 0 : z == g.nz - 1);
+      const float v = feq[(long long)i * g.n + idx] +
+                      (pull_rolled<Q>(fin, g, i, nbx, y, z) - feq[(long long)i * g.n + nb]);
+      f[i] = other ? f[i] : v;
+    });
+  }
+}
+
+template <int Q>
+__global__ void __launch_bounds__(kThreads)
+    k_stream(const __grid_constant__ Geom g, const NodeDecomp dec,
+             const __grid_constant__ StepPlanes p, const float *fin, const float *rho,
+             const float *feq) {
+  chain_enter();
   const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
   if (idx >= (unsigned)g.n) return;
   int x, y, z;
   dec(idx, x, y, z);
-#pragma unroll
-  for (int i = 0; i < Q; ++i) {
-    int fc = -1;
-    if (x == 0 && (V::ex(i) > 0 || g.face[0] == LBM_BC_NON_EQUILIBRIUM)) fc = 0;
-    if (x == g.nx - 1 && (V::ex(i) < 0 || g.face[1] == LBM_BC_NON_EQUILIBRIUM)) fc = 1;
-    if (V::ey(i) > 0 && y == 0) fc = 2;
-    if (V::ey(i) < 0 && y == g.ny - 1) fc = 3;
-    if (V::ez(i) > 0 && z == 0) fc = 4;
-    if (V::ez(i) < 0 && z == g.nz - 1) fc = 5;
-    float v;
-    if (fc < 0) {
-      v = fin[(long long)i * g.n + idx - ((long long)V::ex(i) * g.nyz + (long long)V::ey(i) * g.nz +
-                                          V::ez(i))];
-    } else {
-      const int code = g.face[fc];
-      if (code == LBM_BC_PERIODICAL) {
-        int sx = x, sy = y, sz = z;
-        const bool first = (fc & 1) == 0;
-        if ((fc >> 1) == 0) sx = first ? g.nx - 1 : 0;
-        else if ((fc >> 1) == 1) sy = first ? g.ny - 1 : 0;
-        else sz = first ? g.nz - 1 : 0;
-        v = fin[(long long)i * g.n + ((long long)sx * g.ny + sy) * g.nz + sz];
-      } else if (code == LBM_BC_NON_EQUILIBRIUM) {
-        const int nbx = fc == 0 ? 1 : g.nx - 2;
-        const long long nb = ((long long)nbx * g.ny + y) * g.nz + z;
-        const float rolled = pull_rolled<Q>(fin, g, i, nbx, y, z);
-        v = feq[(long long)i * g.n + idx] + (rolled - feq[(long long)i * g.n + nb]);
-      } else {
-        v = fin[(long long)V::rev(i) * g.n + idx];
-        if (code == LBM_BC_WALL_WITH_SPEED) {
-          const float eu = (float)V::ex(i) * g.uw[fc][0] + (float)V::ey(i) * g.uw[fc][1] +
-                           (float)V::ez(i) * g.uw[fc][2];
-          v -= 2.f * (rho[idx] * V::w(i)) * eu * g.inv_cs2;
-        }
-      }
-    }
-    fout[(long long)i * g.n + idx] = v;
-  }
+  float f[Q];
+  stream_node<Q>(p, g, fin, rho, feq, idx, x, y, z, f);
+  static_for<Q>([&](auto ic) {
+    constexpr int i = decltype(ic)::value;
+    static_cast<float *>(p.dst[i])[idx] = f[i];
+  });
 }
 
 __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
   if (v >= 0.f) atomicMax(reinterpret_cast<int *>(addr), __float_as_int(v));
 }
 
+// Moments of one node to the fields, and the block's greatest density to rmax.
+// Called by every thread of the block (inside: the node exists).
 template <int Q>
-__global__ void __launch_bounds__(kThreads)
-    k_moments(const Geom g, const NodeDecomp dec, const float *f, const float *fol, float *rho,
-              float *u, float *p, float *rmax) {
+__device__ __forceinline__ void write_moments(const Geom &g, bool inside, const float f[Q],
+                                              const float *fol, unsigned idx, int x, int y, int z,
+                                              float *rho, float *u, float *p, float *rmax) {
   __shared__ float s_max[kThreads / 32];
-  const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
   float r = 0.f;
-  if (idx < (unsigned)g.n) {
-    int x, y, z;
-    dec(idx, x, y, z);
-    float fl[Q];
-#pragma unroll
-    for (int i = 0; i < Q; ++i) fl[i] = f[(long long)i * g.n + idx];
+  if (inside) {
     const float fx = fol ? fol[3ull * idx] : 0.f, fy = fol ? fol[3ull * idx + 1] : 0.f,
                 fz = fol ? fol[3ull * idx + 2] : 0.f;
     float ux, uy, uz;
-    moments<Q>(fl, fx, fy, fz, on_any_face(g, x, y, z), r, ux, uy, uz);
+    moments<Q>(f, fx, fy, fz, on_any_face(g, x, y, z), r, ux, uy, uz);
     rho[idx] = r;
     if (p != nullptr) p[idx] = r / 3.0f;
     u[3ull * idx] = ux;
@@ -172,10 +174,51 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+template <int Q>
+__global__ void __launch_bounds__(kThreads)
+    k_moments(const Geom g, const NodeDecomp dec, const float *f, const float *fol, float *rho,
+              float *u, float *p, float *rmax) {
+  chain_enter();
+  const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
+  const bool inside = idx < (unsigned)g.n;
+  int x = 0, y = 0, z = 0;
+  float fl[Q];
+  if (inside) {
+    dec(idx, x, y, z);
+#pragma unroll
+    for (int i = 0; i < Q; ++i) fl[i] = f[(long long)i * g.n + idx];
+  }
+  write_moments<Q>(g, inside, fl, fol, idx, x, y, z, rho, u, p, rmax);
+}
+
+// f_stream and the update_u_rou after it in one pass: the streamed
+// populations are still in registers when their moments are taken.
+template <int Q>
+__global__ void __launch_bounds__(kThreads)
+    k_stream_moments(const __grid_constant__ Geom g, const NodeDecomp dec,
+                     const __grid_constant__ StepPlanes pl, const float *fin, const float *feq,
+                     const float *fol, float *rho, float *u, float *p, float *rmax) {
+  chain_enter();
+  const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
+  const bool inside = idx < (unsigned)g.n;
+  int x = 0, y = 0, z = 0;
+  float f[Q];
+  if (inside) {
+    dec(idx, x, y, z);
+    stream_node<Q>(pl, g, fin, rho, feq, idx, x, y, z, f);
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      static_cast<float *>(pl.dst[i])[idx] = f[i];
+    });
+  }
+  write_moments<Q>(g, inside, f, fol, idx, x, y, z, rho, u, p, rmax);
+}
+
 // update_u_rou_boundary's NON_EQUILIBRIUM part (flow/d3/base.py:135-148): the
 // inlet takes the duct profile scaled by Re mu / max(rho) / min(Y, Z) and the
 // density of plane 1; the outlet copies plane X-2.  One thread per (y, z).
 __global__ void k_neq_moments(const Geom g, float *rho, float *u, const float *rmax) {
+  chain_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nyz) return;
   const long long plane = g.nyz;
@@ -194,6 +237,7 @@ __global__ void k_neq_moments(const Geom g, float *rho, float *u, const float *r
 template <int Q>
 __global__ void __launch_bounds__(kThreads)
     k_force(const Geom g, float *f, const float *u, const float *fol) {
+  chain_enter();
   const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
   if (idx >= (unsigned)g.n) return;
   float fl[Q];
@@ -246,9 +290,10 @@ struct RunInit {
 
 template <int Q>
 struct RunCollide {
-  static int run(const Geom &g, float *f, const float *rho, const float *u, float *feq,
+  static int run(const Geom &g, float *f, const float *rho, const float *u, float *feq, float *rmax,
                  cudaStream_t s) {
-    k_collide<Q><<<blocks_for(g.n, kThreads), kThreads, 0, s>>>(g, f, rho, u, feq);
+    launch_chained(k_collide<Q>, blocks_for(g.n, kThreads), kThreads, 0, s, g, f, rho, u, feq,
+                   rmax);
     LBM_LAUNCH_CHECK("lbm_collide");
     return LBM_OK;
   }
@@ -258,9 +303,24 @@ template <int Q>
 struct RunStream {
   static int run(const Geom &g, const float *fin, float *fout, const float *rho, const float *feq,
                  cudaStream_t s) {
-    k_stream<Q><<<blocks_for(g.n, kThreads), kThreads, 0, s>>>(g, make_decomp(g), fin, fout, rho,
-                                                               feq);
+    StepPlanes p;
+    fill_step_planes(g, Q, LBM_STORAGE_FP32, fin, fout, p);
+    launch_chained(k_stream<Q>, blocks_for(g.n, kThreads), kThreads, 0, s, g, make_decomp(g), p,
+                   fin, rho, feq);
     LBM_LAUNCH_CHECK("lbm_stream");
+    return LBM_OK;
+  }
+};
+
+template <int Q>
+struct RunStreamMoments {
+  static int run(const Geom &g, const float *fin, float *fout, const float *feq, const float *fol,
+                 float *rho, float *u, float *p, float *rmax, cudaStream_t s) {
+    StepPlanes pl;
+    fill_step_planes(g, Q, LBM_STORAGE_FP32, fin, fout, pl);
+    launch_chained(k_stream_moments<Q>, blocks_for(g.n, kThreads), kThreads, 0, s, g,
+                   make_decomp(g), pl, fin, feq, fol, rho, u, p, rmax);
+    LBM_LAUNCH_CHECK("lbm_compute_flow");
     return LBM_OK;
   }
 };
@@ -269,8 +329,8 @@ template <int Q>
 struct RunMoments {
   static int run(const Geom &g, const float *f, const float *fol, float *rho, float *u, float *p,
                  float *rmax, cudaStream_t s) {
-    k_moments<Q><<<blocks_for(g.n, kThreads), kThreads, 0, s>>>(g, make_decomp(g), f, fol, rho, u,
-                                                                p, rmax);
+    launch_chained(k_moments<Q>, blocks_for(g.n, kThreads), kThreads, 0, s, g, make_decomp(g), f,
+                   fol, rho, u, p, rmax);
     LBM_LAUNCH_CHECK("lbm_moments");
     return LBM_OK;
   }
@@ -279,7 +339,7 @@ struct RunMoments {
 template <int Q>
 struct RunForce {
   static int run(const Geom &g, float *f, const float *u, const float *fol, cudaStream_t s) {
-    k_force<Q><<<blocks_for(g.n, kThreads), kThreads, 0, s>>>(g, f, u, fol);
+    launch_chained(k_force<Q>, blocks_for(g.n, kThreads), kThreads, 0, s, g, f, u, fol);
     LBM_LAUNCH_CHECK("lbm_add_force");
     return LBM_OK;
   }
@@ -469,7 +529,8 @@ int lbm_collide(const lbm_lattice *lat, float *f, const float *rho, const float 
     set_error("lbm_collide: f, rho and u are required");
     return LBM_ERR_INVALID;
   }
-  return dispatch_q<RunCollide>(lat->q, make_geom(lat), f, rho, u, feq, (cudaStream_t)stream);
+  return dispatch_q<RunCollide>(lat->q, make_geom(lat), f, rho, u, feq, static_cast<float *>(nullptr),
+                                (cudaStream_t)stream);
 }
 
 int lbm_stream(const lbm_lattice *lat, const float *f_in, float *f_out, const float *rho,
@@ -522,8 +583,37 @@ int lbm_moments(const lbm_lattice *lat, const float *f, const float *fol, float 
   }
   rc = dispatch_q<RunMoments>(lat->q, g, f, fol, rho, u, p, neq_in ? scratch : nullptr, s);
   if (rc || !neq) return rc;
-  k_neq_moments<<<blocks_for(g.nyz, 128), 128, 0, s>>>(g, rho, u, scratch);
+  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch);
   LBM_LAUNCH_CHECK("lbm_moments");
+  return LBM_OK;
+}
+
+int lbm_compute_flow(const lbm_lattice *lat, float *f, float *f_out, const float *fol, float *rho,
+                     float *u, float *p, float *feq, float *scratch, void *stream) {
+  int rc = check_lattice(lat);
+  if (rc) return rc;
+  if (lat->pz != 0 && lat->pz != lat->nz) {
+    set_error("lbm_compute_flow: the single-function calls take dense arrays (pz = 0 or nz)");
+    return LBM_ERR_INVALID;
+  }
+  if (f == nullptr || f_out == nullptr || f == f_out || rho == nullptr || u == nullptr ||
+      feq == nullptr || scratch == nullptr) {
+    set_error("lbm_compute_flow: distinct f and f_out, rho, u, feq and one float of scratch are "
+              "required");
+    return LBM_ERR_INVALID;
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  const Geom g = make_geom(lat);
+  rc = dispatch_q<RunCollide>(lat->q, g, f, static_cast<const float *>(rho),
+                              static_cast<const float *>(u), feq, scratch, s);
+  if (rc) return rc;
+  const bool neq_in = lat->face[0] == LBM_BC_NON_EQUILIBRIUM;
+  rc = dispatch_q<RunStreamMoments>(lat->q, g, static_cast<const float *>(f), f_out,
+                                    static_cast<const float *>(feq), fol, rho, u, p,
+                                    neq_in ? scratch : nullptr, s);
+  if (rc || !any_face(lat, LBM_BC_NON_EQUILIBRIUM)) return rc;
+  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch);
+  LBM_LAUNCH_CHECK("lbm_compute_flow");
   return LBM_OK;
 }
 

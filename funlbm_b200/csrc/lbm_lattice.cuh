@@ -490,6 +490,7 @@ struct StepPlanes {
 template <typename R>
 struct WallRho {
   R v[3];
+  __device__ __forceinline__ explicit WallRho(R rho) : v{rho, rho, rho} {}
   __device__ __forceinline__ WallRho(const Geom &g, const R *__restrict__ face_rho,
                                      const RowFaces &r, int x, int y, int z) {
     auto at = [&](int fc, bool on) {
@@ -531,19 +532,17 @@ __device__ __forceinline__ bool on_moving_wall(const Geom &g, const RowFaces &r,
            (z == 0 ? 16u : 0u) | (z == g.nz - 1 ? 32u : 0u)) & g.moving) != 0;
 }
 
-// Pull of one node with the reference's face rules; no branch between the
-// loads, so all Q of them issue together.  WORK: working values (d for the
-// shifted storages) as the fused step uses them; otherwise f.
+// Pull of one node with the reference's face rules but for the moving walls'
+// correction; no branch between the loads, so all Q of them issue together.
+// WORK: working values (d for the shifted storages) as the fused step uses
+// them; otherwise f.
 template <int Q, int S, bool WORK>
-__device__ __forceinline__ void pull_node(const StepPlanes &p, const Geom &g,
-                                          const typename Storage<S>::R *__restrict__ face_rho,
-                                          unsigned idx, int x, int y, int z,
-                                          typename Storage<S>::R f[Q]) {
+__device__ __forceinline__ void pull_sources(const StepPlanes &p, const Geom &g, const RowFaces &r,
+                                             unsigned idx, int z, typename Storage<S>::R f[Q]) {
   using St = Storage<S>;
   using T = typename St::T;
   using V = VSet<Q>;
   const bool bottom = z == 0, top = z == g.nz - 1;
-  const RowFaces r(g, x, y);
   auto pull = [&](auto ic, const T *ps, bool shifted) {
     constexpr int i = decltype(ic)::value;
     constexpr int ez = V::ez(i);
@@ -572,9 +571,19 @@ __device__ __forceinline__ void pull_node(const StepPlanes &p, const Geom &g,
       pull(ic, static_cast<const T *>(src[i]) + idx, !enters<V::ex(i), V::ey(i)>(r));
     });
   }
+}
+
+// Pull of one node with all of the reference's face rules.
+template <int Q, int S, bool WORK>
+__device__ __forceinline__ void pull_node(const StepPlanes &p, const Geom &g,
+                                          const typename Storage<S>::R *__restrict__ face_rho,
+                                          unsigned idx, int x, int y, int z,
+                                          typename Storage<S>::R f[Q]) {
+  const RowFaces r(g, x, y);
+  pull_sources<Q, S, WORK>(p, g, r, idx, z, f);
   if (on_moving_wall(g, r, z)) {
-    constexpr int kSh = WORK ? St::kShift : 0;
-    const WallRho<typename St::R> rho(g, face_rho, r, x, y, z);
+    constexpr int kSh = WORK ? Storage<S>::kShift : 0;
+    const WallRho<typename Storage<S>::R> rho(g, face_rho, r, x, y, z);
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       if constexpr (i != 0) f[i] -= moving_wall<Q, i, kSh>(g, rho, r, z);

@@ -173,6 +173,8 @@ class FlowD3(Flow):
         self._last_fields = ()
         self._tau_t = None
         self._x = None
+        self._fp64 = False
+        self._fol_zero = False      # FOL is known to be zero everywhere
 
     # -- geometry ------------------------------------------------------------
     @property
@@ -218,6 +220,7 @@ class FlowD3(Flow):
         self._rou = torch.ones((X, Y, Z, 1), device=dev)
         self._p = torch.zeros((X, Y, Z, 1), device=dev)
         self._FOL = torch.zeros((X, Y, Z, 3), device=dev)
+        self._fol_zero = True
         self._scratch = torch.zeros(1, device=dev)
         self._mode = "ref"
         self._obs_valid = True
@@ -329,6 +332,7 @@ class FlowD3(Flow):
         if "_p" in need:
             self._p = self._rou / 3.0
         if "_FOL" in need:
+            self._fol_zero = False
             new_field, new_uniform = fields
             rdt = lat.real_dtype
             # the uniform force reaches the kernels as float32
@@ -437,6 +441,29 @@ class FlowD3(Flow):
         call("lbm_moments", ctypes_ref(self._lat.desc_fp32), ptr(self._f), ptr(self._FOL),
              ptr(self._rou), ptr(self._u), ptr(self._p), ptr(self._scratch), self._lat.stream())
 
+    # the methods that one step of the reference's call sequence runs
+    _STEP_METHODS = ("cul_equ", "f_stream", "update_u_rou", "cul_equ2")
+
+    def _plain_methods(self):
+        """Whether the step methods are this class's own (a subclass or an
+        instance may replace them, and is then called one by one)."""
+        cls = type(self)
+        return not self._fp64 and all(
+            getattr(cls, k) is getattr(FlowD3, k) and k not in self.__dict__
+            for k in self._STEP_METHODS)
+
+    def compute_flow(self, step=0):
+        """cul_equ, f_stream and update_u_rou in one call (lbm/base.py:159-163)."""
+        self._to_ref()
+        if self._feq is None:
+            self._feq = torch.empty_like(self._f)
+        if self._f2 is None:
+            self._f2 = torch.empty_like(self._f)
+        call("lbm_compute_flow", ctypes_ref(self._lat.desc_fp32), ptr(self._f), ptr(self._f2),
+             ptr(self._FOL), ptr(self._rou), ptr(self._u), ptr(self._p), ptr(self._feq),
+             ptr(self._scratch), self._lat.stream())
+        self._f, self._f2 = self._f2, self._f
+
     def update_u_rou_boundary(self, *args, **kwargs):
         """Included in update_u_rou (the moment kernel applies the face rules)."""
         self.update_u_rou()
@@ -501,10 +528,12 @@ class FlowD3(Flow):
 
     @property
     def FOL(self):
+        self._fol_zero = False      # (the caller may write to it)
         return self._get("_FOL")
 
     @FOL.setter
     def FOL(self, value):
+        self._fol_zero = False
         self._set("_FOL", torch.as_tensor(value, dtype=torch.float32, device=self.device)
                   .reshape(self.shape + (3,)).contiguous())
 

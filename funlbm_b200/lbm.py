@@ -280,11 +280,23 @@ class LBMBase:
 
     # -- reference call sequence -----------------------------------------------
     def _compute_flow(self) -> None:
+        if self.flow._plain_methods():
+            self.flow.compute_flow(step=self.step)
+            return
         self.flow.cul_equ(step=self.step)
         self.flow.f_stream()
         self.flow.update_u_rou(step=self.step)
 
+    def _no_force(self):
+        """Whether this step has no force anywhere, before and after: no
+        particles, no body force, FOL zero since the last step.  cul_equ2 then
+        adds zeros and the second update_u_rou repeats the first.  (Not when a
+        subclass or an instance replaces one of the methods.)"""
+        return False
+
     def _handle_immersed_boundary(self) -> None:
+        if self._no_force():
+            return
         self.flow_to_lagrange()
         self.particle_to_wall()
         for particle in self.particle_swarm.particles:
@@ -518,6 +530,15 @@ class LBMD3(LBMBase):
             self._fi ^= 1
         self._g_old = plan["g_new"]
 
+    _COUPLING = ("flow_to_lagrange", "particle_to_wall", "lagrange_to_flow")
+
+    def _no_force(self):
+        cls = type(self)
+        return (not self.particle_swarm.particles and self.body_force == (0.0, 0.0, 0.0)
+                and self.flow._fol_zero and self.flow._plain_methods()
+                and all(getattr(cls, k) is getattr(LBMD3, k) and k not in self.__dict__
+                        for k in self._COUPLING))
+
     # -- reference-mode IBM methods (lbm/lbm3d.py:66-167) -------------------------
     def flow_to_lagrange(self, *args, **kwargs):
         parts = self.particle_swarm.particles
@@ -541,6 +562,7 @@ class LBMD3(LBMBase):
         fl = self.flow
         fl._to_ref()
         fl._FOL.zero_()
+        fl._fol_zero = not self.particle_swarm.particles and self.body_force == (0.0, 0.0, 0.0)
         parts = self.particle_swarm.particles
         if parts:
             if not hasattr(self, "_ref_chunks"):
