@@ -116,6 +116,8 @@ SIGNATURES = {
     "lbm_collide": (I, [_LAT, _P, _P, _P, _P, _P]),
     "lbm_stream": (I, [_LAT, _P, _P, _P, _P, _P]),
     "lbm_moments": (I, [_LAT, _P, _P, _P, _P, _P, _P, _P]),
+    "lbm_coupled_step": (I, [_LAT, _P, _P, _FORCE, _P, _P, _PART, F, F, F, F, ctypes.c_int32, _P,
+                             _P, _P, _P]),
     "lbm_compute_flow": (I, [_LAT, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "lbm_add_force": (I, [_LAT, _P, _P, _P, _P]),
     "ibm_interpolate": (I, [_LAT, _P, _FORCE, _P, _P, _P, _PART, F, ctypes.c_int32, _P, _P]),
@@ -179,14 +181,22 @@ def check(rc, what=""):
 
 
 def call(name, *args):
-    rc = getattr(load(), name)(*args)
-    check(rc, name)
+    rc = getattr(_lib or load(), name)(*args)
+    if rc != LBM_OK:
+        check(rc, name)
 
 
 def ptr(t):
     """Device address of a tensor (None for None)."""
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def stream_of(torch_mod, device=None):
-    return ctypes.c_void_p(torch_mod.cuda.current_stream(device).cuda_stream)
+    """Handle of the current CUDA stream of `device` (a torch.device; None or
+    one without an index: the current device)."""
+    index = getattr(device, "index", None)
+    if index is None:
+        if device is not None and not isinstance(device, torch_mod.device):
+            return torch_mod.cuda.current_stream(device).cuda_stream
+        index = torch_mod.cuda.current_device()
+    return torch_mod._C._cuda_getCurrentRawStream(index)

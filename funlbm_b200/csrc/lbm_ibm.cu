@@ -1286,6 +1286,28 @@ int rigid_step(const lbm_particles *pt, float dt, float gl, float rouf, void *st
   return LBM_OK;
 }
 
+int lbm_coupled_step(const lbm_lattice *lat, const void *fa, void *fb, const lbm_force *force,
+                     const float *face_rho_in, float *face_rho_out, const lbm_particles *pt,
+                     float dt, float dx, float gl, float rouf, int32_t step, int32_t *owner,
+                     uint32_t *ibm_status, uint32_t *status, void *stream) {
+  int rc = check_particles(pt, "lbm_coupled_step");
+  if (rc) return rc;
+  if (pt->n_particles > 0) {
+    if (force == nullptr || force->new_field == nullptr || force->new_chunks == nullptr) {
+      set_error("lbm_coupled_step: particles need the new force field and its chunks");
+      return LBM_ERR_INVALID;
+    }
+    float *field = const_cast<float *>(force->new_field);
+    uint8_t *chunks = const_cast<uint8_t *>(force->new_chunks);
+    rc = ibm_interpolate_wall_claim(lat, fa, force, face_rho_in, pt, dt, dx, step, ibm_status,
+                                    field, chunks, owner, stream);
+    if (rc) return rc;
+    if ((rc = ibm_spread_claimed(lat, pt, field, chunks, owner, stream))) return rc;
+    if ((rc = rigid_step(pt, dt, gl, rouf, stream))) return rc;
+  }
+  return lbm_flow_step(lat, fa, fb, force, face_rho_in, face_rho_out, nullptr, status, stream);
+}
+
 int rigid_extremes(const lbm_particles *pt, void *stream) {
   int rc = check_particles(pt, "rigid_extremes");
   if (rc) return rc;

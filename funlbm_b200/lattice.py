@@ -10,6 +10,7 @@ bfloat16); fp64 buffers hold f.  Everything numeric runs in ``liblbm_b200.so``.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import numpy as np
@@ -251,21 +252,11 @@ class Lattice:
 
 def make_force(old_uniform=(0, 0, 0), new_uniform=(0, 0, 0), old_field=None, new_field=None,
                old_chunks=None, new_chunks=None):
-    f = LbmForce()
-    for k in range(3):
-        f.old_uniform[k] = float(old_uniform[k])
-        f.new_uniform[k] = float(new_uniform[k])
-    f.old_field = None if old_field is None else old_field.data_ptr()
-    f.new_field = None if new_field is None else new_field.data_ptr()
-    f.old_chunks = None if old_chunks is None else old_chunks.data_ptr()
-    f.new_chunks = None if new_chunks is None else new_chunks.data_ptr()
-    return f
+    return LbmForce(tuple(old_uniform), tuple(new_uniform), ptr(old_field), ptr(new_field),
+                    ptr(old_chunks), ptr(new_chunks))
 
 
-def ctypes_ref(s):
-    import ctypes
-
-    return ctypes.byref(s)
+ctypes_ref = ctypes.byref
 
 
 _WCACHE = {}
