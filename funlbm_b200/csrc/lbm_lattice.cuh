@@ -350,16 +350,38 @@ struct F2 {
   __device__ __forceinline__ F2(float a, float b) : v(make_float2(a, b)) {}
   __device__ __forceinline__ explicit F2(float2 p) : v(p) {}
 };
-__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return F2(__fadd2_rn(a.v, b.v)); }
-__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return F2(__fmul2_rn(a.v, b.v)); }
+__device__ __forceinline__ unsigned long long f2_bits(F2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.v.x), "f"(a.v.y));
+  return r;
+}
+__device__ __forceinline__ F2 f2_of(unsigned long long r) {
+  F2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.v.x), "=f"(a.v.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ F2 fma_rn(F2 a, F2 b, F2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;"
+      : "=l"(r)
+      : "l"(f2_bits(a)), "l"(f2_bits(b)), "l"(f2_bits(c)));
+  return f2_of(r);
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2_bits(a)), "l"(f2_bits(b)));
+  return f2_of(r);
+}
+// a b as a b + 0: the assembler contracts a packed multiply followed by a
+// packed add to one fused operation, also where both are written as rounded
+// (add_force's ux fx + uy fy differed from the scalar code in one pair of 2000),
+// but not this form.  The same value; only a product of -0 becomes +0.
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fma_rn(a, b, F2(0.f)); }
 __device__ __forceinline__ F2 operator-(F2 a) { return F2(-a.v.x, -a.v.y); }
 // a - b as a + (-1) b: one rounding, as the subtraction
-__device__ __forceinline__ F2 operator-(F2 a, F2 b) {
-  return F2(__ffma2_rn(b.v, make_float2(-1.f, -1.f), a.v));
-}
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return fma_rn(b, F2(-1.f), a); }
 __device__ __forceinline__ F2 &operator+=(F2 &a, F2 b) { return a = a + b; }
 __device__ __forceinline__ F2 &operator-=(F2 &a, F2 b) { return a = a - b; }
-__device__ __forceinline__ F2 fma_rn(F2 a, F2 b, F2 c) { return F2(__ffma2_rn(a.v, b.v, c.v)); }
 __device__ __forceinline__ float recip(float x) { return 1.f / x; }
 __device__ __forceinline__ F2 recip(F2 x) { return F2(1.f / x.v.x, 1.f / x.v.y); }
 // u, zero where the node lies on a boundary plane
