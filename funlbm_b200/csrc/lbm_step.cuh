@@ -374,27 +374,60 @@ __device__ __forceinline__ double from_ordered_bits(unsigned long long o) {
   return __longlong_as_double((long long)b);
 }
 
+// Per-thread accumulators: extremes in the arithmetic type (exact), sums in
+// double.
+template <typename R>
 struct StatAcc {
-  double mn[3], sm[3], mx[3];
+  R mn[3], mx[3];
+  double sm[3];
 };
 
-__device__ __forceinline__ void stat_add(StatAcc &s, int k, double v) {
-  s.mn[k] = fmin(s.mn[k], v);
-  s.mx[k] = fmax(s.mx[k], v);
-  s.sm[k] += v;
+// sum of v[0..N) as a rounded sum and its error, added to `acc`.  The
+// conversion of every value to double was what bounded the kernel (a quarter
+// of the float64 rate): here each addition's error is recovered in float32
+// (|s| >= |v|: the rest population comes first and is the largest) and two
+// values are converted per node.
+template <int N>
+__device__ __forceinline__ void add_all(const float v[N], double &acc) {
+  float s = v[0], e = 0.f;
+#pragma unroll
+  for (int i = 1; i < N; ++i) {
+    const float t = s + v[i];
+    e += v[i] - (t - s);
+    s = t;
+  }
+  acc += (double)s;
+  if (fabsf(s) < 3.0e38f) acc += (double)e;   // (an infinite sum has no error term)
+}
+template <int N>
+__device__ __forceinline__ void add_all(const double v[N], double &acc) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) acc += v[i];
 }
 
+// Resident blocks per SM of k_stats, also its grid (5 blocks of D3Q19 spill
+// and take 66.5 us where 4 take 64.5).
+template <int Q, int S>
+constexpr int stats_blocks() {
+  return Storage<S>::kBits == 64 ? 2 : Q == 27 ? 3 : 4;
+}
+
+// Bound by the read of the populations (D3Q19 fp32 193 x 161 x 129: 305 MB, 47
+// us at the copy peak); float32 extremes and the sums above took the registers
+// from 80 to 64 (4 resident blocks instead of 3) and the three launches of
+// lbm_flow_stats from 98 to 65 us.
 template <int Q, int S, bool FORCE>
-__global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__ StepArgs a,
-                                                         unsigned long long *out) {
+__global__ void __launch_bounds__(kStatsThreads, (stats_blocks<Q, S>()))
+    k_stats(const __grid_constant__ StepArgs a, unsigned long long *out) {
+  chain_enter();
   using St = Storage<S>;
   using R = typename St::R;
   using V = VSet<Q>;
-  __shared__ StatAcc sh[kStatsThreads / 32];
-  StatAcc acc;
+  __shared__ StatAcc<R> sh[kStatsThreads / 32];
+  StatAcc<R> acc;
   for (int k = 0; k < 3; ++k) {
-    acc.mn[k] = INFINITY;
-    acc.mx[k] = -INFINITY;
+    acc.mn[k] = R(INFINITY);
+    acc.mx[k] = -R(INFINITY);
     acc.sm[k] = 0.0;
   }
   const R *face_rho = static_cast<const R *>(a.face_rho_in);
@@ -411,22 +444,21 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__
     R rho, drho, ux, uy, uz;
     finish_node_m<Q, FORCE, St::kDev, St::kShift>(a, f, idx, x, y, z, on_any_face(a.g, x, y, z), cf,
                                                   bad, rho, drho, ux, uy, uz);
-    R fmn = R(INFINITY), fmx = -R(INFINITY);
-    double fsum = 0.0;
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
-      const R v = St::kDev ? f[i] * (R(1) / R(1 << St::kShift)) + V::template wr<R>(i) : f[i];
-      fsum += (double)v;
-      fmn = fmin(fmn, v);
-      fmx = fmax(fmx, v);
+      f[i] = St::kDev ? f[i] * (R(1) / R(1 << St::kShift)) + V::template wr<R>(i) : f[i];
+      acc.mn[0] = fmin(acc.mn[0], f[i]);
+      acc.mx[0] = fmax(acc.mx[0], f[i]);
     });
-    acc.mn[0] = fmin(acc.mn[0], (double)fmn);
-    acc.mx[0] = fmax(acc.mx[0], (double)fmx);
-    acc.sm[0] += fsum;
-    stat_add(acc, 1, (double)ux);
-    stat_add(acc, 1, (double)uy);
-    stat_add(acc, 1, (double)uz);
-    stat_add(acc, 2, (double)rho);
+    add_all<Q>(f, acc.sm[0]);
+    acc.mn[1] = fmin(acc.mn[1], fmin(ux, fmin(uy, uz)));
+    acc.mx[1] = fmax(acc.mx[1], fmax(ux, fmax(uy, uz)));
+    acc.sm[1] += (double)ux;
+    acc.sm[1] += (double)uy;
+    acc.sm[1] += (double)uz;
+    acc.mn[2] = fmin(acc.mn[2], rho);
+    acc.mx[2] = fmax(acc.mx[2], rho);
+    acc.sm[2] += (double)rho;
   }
   report_bad(a.status, bad);
   for (int k = 0; k < 3; ++k) {
@@ -439,19 +471,18 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (lane == 0) sh[wid] = acc;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    StatAcc t = sh[0];
-    for (int w = 1; w < kStatsThreads / 32; ++w)
-      for (int k = 0; k < 3; ++k) {
-        t.mn[k] = fmin(t.mn[k], sh[w].mn[k]);
-        t.mx[k] = fmax(t.mx[k], sh[w].mx[k]);
-        t.sm[k] += sh[w].sm[k];
-      }
-    for (int k = 0; k < 3; ++k) {
-      atomicMin(out + 3 * k, ordered_bits(t.mn[k]));
-      atomicAdd(reinterpret_cast<double *>(out + 3 * k + 1), t.sm[k]);
-      atomicMax(out + 3 * k + 2, ordered_bits(t.mx[k]));
+  if (threadIdx.x < 3) {   // thread k: quantity k
+    const int k = threadIdx.x;
+    R mn = sh[0].mn[k], mx = sh[0].mx[k];
+    double sm = sh[0].sm[k];
+    for (int w = 1; w < kStatsThreads / 32; ++w) {
+      mn = fmin(mn, sh[w].mn[k]);
+      mx = fmax(mx, sh[w].mx[k]);
+      sm += sh[w].sm[k];
     }
+    atomicMin(out + 3 * k, ordered_bits((double)mn));
+    atomicAdd(reinterpret_cast<double *>(out + 3 * k + 1), sm);
+    atomicMax(out + 3 * k + 2, ordered_bits((double)mx));
   }
 }
 
@@ -460,6 +491,7 @@ __global__ void __launch_bounds__(kStatsThreads) k_stats(const __grid_constant__
 // that includes this header may carry it)
 template <int Q>
 __global__ void k_stats_init(unsigned long long *out) {
+  chain_enter();
   const int k = threadIdx.x;
   if (k >= 9) return;
   const int c = k % 3;
@@ -470,6 +502,7 @@ __global__ void k_stats_init(unsigned long long *out) {
 // in place: keys -> min / max, sums -> means over n*q, 3n and n values
 template <int Q>
 __global__ void k_stats_finish(unsigned long long *out, double n) {
+  chain_enter();
   const int k = threadIdx.x;
   if (k >= 9) return;
   const int c = k % 3;
@@ -1292,13 +1325,13 @@ int run_stats_qs(const StepArgs &a, bool force, unsigned long long *out, cudaStr
   int sms = 148;
   if (device_info(d)) sms = d.sms;
   const unsigned blocks = (unsigned)std::min<long long>(blocks_for(a.g.n, kStatsThreads),
-                                                        (long long)sms * 8);
-  k_stats_init<Q><<<1, 32, 0, s>>>(out);
+                                                        (long long)sms * stats_blocks<Q, S>());
+  launch_chained(k_stats_init<Q>, 1, 32, 0, s, out);
   if (force)
-    k_stats<Q, S, true><<<blocks, kStatsThreads, 0, s>>>(a, out);
+    launch_chained(k_stats<Q, S, true>, blocks, kStatsThreads, 0, s, a, out);
   else
-    k_stats<Q, S, false><<<blocks, kStatsThreads, 0, s>>>(a, out);
-  k_stats_finish<Q><<<1, 32, 0, s>>>(out, (double)a.g.n);
+    launch_chained(k_stats<Q, S, false>, blocks, kStatsThreads, 0, s, a, out);
+  launch_chained(k_stats_finish<Q>, 1, 32, 0, s, out, (double)a.g.n);
   LBM_LAUNCH_CHECK("lbm_flow_stats");
   return LBM_OK;
 }
