@@ -188,6 +188,11 @@ def call(name, *args):
 
 def ptr(t):
     """Device address of a tensor (None for None)."""
+    return None if t is None else ctypes.c_void_p(t.data_ptr())
+
+
+def addr(t):
+    """ptr as a plain int, for calls whose argument types are declared."""
     return None if t is None else t.data_ptr()
 
 
@@ -197,6 +202,6 @@ def stream_of(torch_mod, device=None):
     index = getattr(device, "index", None)
     if index is None:
         if device is not None and not isinstance(device, torch_mod.device):
-            return torch_mod.cuda.current_stream(device).cuda_stream
+            return ctypes.c_void_p(torch_mod.cuda.current_stream(device).cuda_stream)
         index = torch_mod.cuda.current_device()
-    return torch_mod._C._cuda_getCurrentRawStream(index)
+    return ctypes.c_void_p(torch_mod._C._cuda_getCurrentRawStream(index))

@@ -378,6 +378,7 @@ static int build_step_args(const lbm_lattice *lat, const void *fa, void *fb, con
       a.gn[k] = force->new_uniform[k];
       use_force = use_force || a.go[k] != 0.f || a.gn[k] != 0.f;
     }
+    a.uniform = use_force;
     a.fol_old = force->old_field;
     a.fol_new = force->new_field;
     a.ch_old = force->old_chunks;

@@ -22,6 +22,7 @@ struct StepArgs {
   const void *fa;
   void *fb;
   float go[3], gn[3];
+  int uniform;       // go or gn is not zero
   // fields, face densities and observation buffers hold the storage's
   // arithmetic type (float64 for LBM_STORAGE_FP64, float32 otherwise)
   const void *fol_old, *fol_new;
@@ -74,54 +75,47 @@ __device__ __forceinline__ ChunkForce chunk_force(const StepArgs &a, unsigned id
   return c;
 }
 
-// Previous / new force at the node: uniform part plus the fields where the
-// node's chunk carries them.
+// Force at the node: the uniform part plus the field where the node's chunk
+// carries it.
 template <typename R>
-__device__ __forceinline__ void node_force(const StepArgs &a, unsigned idx, ChunkForce cf, R fo[3],
-                                           R fn[3]) {
+__device__ __forceinline__ void node_force(const float uniform[3], const void *field, bool here,
+                                           unsigned idx, R F[3]) {
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    fo[k] = a.go[k];
-    fn[k] = a.gn[k];
-  }
-  if (cf.old_here) {
-    const R *fol = static_cast<const R *>(a.fol_old);
+  for (int k = 0; k < 3; ++k) F[k] = uniform[k];
+  if (here) {
+    const R *fol = static_cast<const R *>(field);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) fo[k] += fol[3ull * idx + k];
-  }
-  if (cf.new_here) {
-    const R *fol = static_cast<const R *>(a.fol_new);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) fn[k] += fol[3ull * idx + k];
+    for (int k = 0; k < 3; ++k) F[k] += fol[3ull * idx + k];
   }
 }
 
 // finish_node_m hands the node's end-of-step moments (the second
 // update_u_rou) to the caller; f is left at the end-of-step populations.
+// Where neither step has a force (no uniform part, neither field in the
+// node's chunk) cul_equ2 adds nothing and the second moment pass repeats the
+// first, so both are skipped -- the same rule in every kernel, and a node of a
+// flagged chunk without force of its own gets the same bits either way.  The
+// new force is read only there: kept from the start of the node together with
+// the old one it cost 20 to 28 registers per thread of the pair kernels.
 template <int Q, bool FORCE, bool DEV, int SH, typename R>
 __device__ __forceinline__ void finish_node_m(const StepArgs &a, R f[Q], unsigned idx, int x,
                                               int y, int z, bool face, ChunkForce cf,
                                               unsigned &bad, R &rho, R &drho, R &ux, R &uy, R &uz) {
-  R fo[3] = {R(0), R(0), R(0)}, fn[3] = {R(0), R(0), R(0)};
-  if constexpr (FORCE) node_force<R>(a, idx, cf, fo, fn);
+  R F[3] = {R(0), R(0), R(0)};
+  if constexpr (FORCE) node_force<R>(a.go, a.fol_old, cf.old_here, idx, F);
   if constexpr (DEV) {
-    dev_moments<Q, SH, FORCE>(f, fo[0], fo[1], fo[2], face, rho, drho, ux, uy, uz);
+    dev_moments<Q, SH, FORCE>(f, F[0], F[1], F[2], face, rho, drho, ux, uy, uz);
   } else {
     drho = R(0);
-    moments<Q>(f, fo[0], fo[1], fo[2], face, rho, ux, uy, uz);
+    moments<Q>(f, F[0], F[1], F[2], face, rho, ux, uy, uz);
   }
-  // Where both the previous and this step's force are zero (everywhere
-  // outside the spread chunks when there is no uniform force) cul_equ2 adds
-  // nothing and the second moment pass repeats the first, so such nodes skip
-  // them -- the same rule in every kernel.  (A zero new force alone is not
-  // enough: the second pass drops the previous force from u.)
-  if (FORCE && (fn[0] != R(0) || fn[1] != R(0) || fn[2] != R(0) || fo[0] != R(0) ||
-                fo[1] != R(0) || fo[2] != R(0))) {
-    add_force<Q, SH>(f, a.g, ux, uy, uz, fn[0], fn[1], fn[2]);
+  if (FORCE && (a.uniform || cf.old_here || cf.new_here)) {
+    node_force<R>(a.gn, a.fol_new, cf.new_here, idx, F);
+    add_force<Q, SH>(f, a.g, ux, uy, uz, F[0], F[1], F[2]);
     if constexpr (DEV)
-      dev_moments<Q, SH, true>(f, fn[0], fn[1], fn[2], face, rho, drho, ux, uy, uz);
+      dev_moments<Q, SH, true>(f, F[0], F[1], F[2], face, rho, drho, ux, uy, uz);
     else
-      moments<Q>(f, fn[0], fn[1], fn[2], face, rho, ux, uy, uz);
+      moments<Q>(f, F[0], F[1], F[2], face, rho, ux, uy, uz);
   }
   bad |= bad_bits(rho, ux, uy, uz);
   if (face && a.face_rho_out != nullptr)
@@ -181,26 +175,21 @@ __device__ __forceinline__ void finish_pair(const StepArgs &a, F2 f[Q], unsigned
   face.a = row_face || z == 0 || z == a.g.nz - 1;
   face.b = row_face || z + 1 == a.g.nz - 1;
   F2 rho, drho, ux, uy, uz;
-  F2 fo[3] = {F2(0.f), F2(0.f), F2(0.f)}, fn[3] = {F2(0.f), F2(0.f), F2(0.f)};
-  if constexpr (FORCE) {
-    float o0[3], n0[3], o1[3], n1[3];
-    node_force<float>(a, idx, c0, o0, n0);
-    node_force<float>(a, two ? idx + 1 : idx, two ? c1 : c0, o1, n1);
+  F2 F[3] = {F2(0.f), F2(0.f), F2(0.f)};
+  auto force = [&](const float uniform[3], const void *field, bool here0, bool here1) {
+    float p[3], q[3];
+    node_force<float>(uniform, field, here0, idx, p);
+    node_force<float>(uniform, field, here1 && two, idx + 1, q);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      fo[k] = F2(o0[k], o1[k]);
-      fn[k] = F2(n0[k], n1[k]);
-    }
-  }
-  dev_moments<Q, SH, FORCE>(f, fo[0], fo[1], fo[2], face, rho, drho, ux, uy, uz);
+    for (int k = 0; k < 3; ++k) F[k] = F2(p[k], q[k]);
+  };
+  if constexpr (FORCE) force(a.go, a.fol_old, c0.old_here, c1.old_here);
+  dev_moments<Q, SH, FORCE>(f, F[0], F[1], F[2], face, rho, drho, ux, uy, uz);
   if constexpr (FORCE) {
-    bool any = false;
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-      any = any || fo[k].v.x != 0.f || fo[k].v.y != 0.f || fn[k].v.x != 0.f || fn[k].v.y != 0.f;
-    if (any) {   // (a node without force next to one that has some is left unchanged by both)
-      add_force<Q, SH>(f, a.g, ux, uy, uz, fn[0], fn[1], fn[2]);
-      dev_moments<Q, SH, true>(f, fn[0], fn[1], fn[2], face, rho, drho, ux, uy, uz);
+    if (a.uniform || c0.old_here || c0.new_here || c1.old_here || c1.new_here) {
+      force(a.gn, a.fol_new, c0.new_here, c1.new_here);
+      add_force<Q, SH>(f, a.g, ux, uy, uz, F[0], F[1], F[2]);
+      dev_moments<Q, SH, true>(f, F[0], F[1], F[2], face, rho, drho, ux, uy, uz);
     }
   }
   bad |= bad_bits(rho.v.x, ux.v.x, uy.v.x, uz.v.x);
@@ -295,7 +284,6 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
   using T = typename St::T;
   if (idx >= (unsigned)a.g.n) return;
   int x, y, z;
-  const ChunkForce cf = chunk_force<FORCE>(a, idx);
   a.dec(idx, x, y, z);
   const unsigned pidx = (unsigned)(x * a.g.ny + y) * (unsigned)a.g.pz + (unsigned)z;
   if (!lbm_in(x < a.g.nx && y < a.g.ny && z < a.g.nz && pidx < (unsigned)a.g.np)) return;
@@ -303,6 +291,7 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
   const R *face_rho = static_cast<const R *>(a.face_rho_in);
   R f[Q];
   pull_node<Q, S, true>(a.p, a.g, face_rho, pidx, x, y, z, f);
+  const ChunkForce cf = chunk_force<FORCE>(a, idx);   // (after the loads, see step_pairs_at)
   unsigned bad = 0;
   finish_node<Q, FORCE, St::kDev, St::kShift, OP>(a, f, idx, x, y, z, on_any_face(a.g, x, y, z), cf,
                                                   bad);
@@ -589,12 +578,6 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
   if (!lbm_in(x < a.g.nx && y < a.g.ny && pidx0 + NZ <= (unsigned)a.g.np &&
               idx0 + nv <= (unsigned)a.g.n))
     return;
-  // (a thread's nodes may lie in two force chunks: dense rows of any length)
-  const ChunkForce cf0 = chunk_force<FORCE>(a, idx0);
-  ChunkForce cf1 = cf0;
-  if constexpr (FORCE) {
-    if (((idx0 + nv - 1) >> 5) != (idx0 >> 5)) cf1 = chunk_force<FORCE>(a, idx0 + nv - 1);
-  }
   const bool bottom = z0 == 0, top = z0 + NZ >= a.g.nz;
   const RowFaces rf(a.g, x, y);
   const void *const *src = a.p.src[rf.cls()];
@@ -646,6 +629,15 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
           in[i].extra = St::raw(static_cast<const T *>(src[i]) + pidx0 + NZ);
       });
     }
+  }
+  // A thread's nodes may lie in two force chunks (dense rows of any length).
+  // The flags are read after the population loads are issued: the branches
+  // here wait for them, and ahead of the loads that wait was a memory round
+  // trip of its own (forced D3Q27 257 x 129 x 129: 212 -> 161 us).
+  const ChunkForce cf0 = chunk_force<FORCE>(a, idx0);
+  ChunkForce cf1 = cf0;
+  if constexpr (FORCE) {
+    if (((idx0 + nv - 1) >> 5) != (idx0 >> 5)) cf1 = chunk_force<FORCE>(a, idx0 + nv - 1);
   }
   Words<kWords> out[OP == Op::kStep ? Q : 1];
 #pragma unroll
@@ -801,11 +793,15 @@ __device__ __forceinline__ void step_vec_body(const StepArgs &a, const unsigned 
 // resident (measured on B200 at 256^3, unforced, 128 threads, fraction of the
 // copy peak without / with the cap: D3Q13 4 nodes 0.915 / 0.927, D3Q15 bf16s
 // 4 nodes - / 0.873, D3Q19 4 nodes 0.687 / 0.859, D3Q27 2 nodes 0.821 /
-// 0.828).  FP32 runs uncapped.
+// 0.828).  FP32 runs uncapped but for the forced D3Q19 pairs (the sphere
+// case's step: 94 registers 19.0 us, 80 17.8; D3Q27 is faster uncapped, 161
+// against 165 us on 257 x 129 x 129).
 template <int Q, int S, int NZ, bool FORCE>
 constexpr int vec_reg_cap() {
+  if (Storage<S>::kBits == 32) return FORCE && NZ == 2 && Q == 19 ? 80 : 0;
   if (Storage<S>::kBits != 16) return 0;
-  if (NZ == 2) return Q == 27 ? 96 : FORCE && Q == 19 ? 80 : 0;
+  if (NZ == 2 && FORCE) return Q == 19 ? 72 : Q == 27 ? 96 : 0;
+  if (NZ == 2) return Q == 27 ? 96 : 0;
   if (NZ == 4) return Q == 13 ? 96 : Q == 15 || Q == 19 ? 128 : 0;
   return 0;
 }
@@ -1279,11 +1275,12 @@ struct StepLauncher {
       // (512^3 3007 us a step; one node per thread is 1 % slower); 16-bit
       // D3Q13 0.83 / 0.93; D3Q15 fp16s 0.83 / 0.77, bf16s 0.82 / 0.87; D3Q19
       // fp16s 0.87 / 0.86 (512^3 0.88 / 0.89), bf16s 0.87 / 0.95; D3Q27 fp16s
-      // 0.83 / 0.82.  Forced kernels keep pairs (4 nodes spill).  Rows of odd
-      // length without pitch take one node per thread; the odd-row pair kernel
-      // is a tuner candidate only.
+      // 0.83 / 0.82.  Padded rows keep pairs but for D3Q13 (D3Q19 fp16s 257^3
+      // 240 us with pairs, 267 with 4 nodes; D3Q13 170, 162), and so do forced
+      // kernels (4 nodes spill).  Rows of odd length without padding take one
+      // node per thread; the odd-row pair kernel is a tuner candidate only.
       constexpr bool four = bits == 16 && (Q == 13 || Q == 19 || (Q == 15 && S == LBM_STORAGE_BF16S));
-      const int want = four && !force ? 4 : 2;
+      const int want = four && !force && (Q == 13 || a.g.pz == a.g.nz) ? 4 : 2;
       nodes = step_shape_ok(want, a.g.pz, bits) ? want : step_shape_ok(2, a.g.pz, bits) ? 2 : 1;
       threads = threads ? threads : 128;
     }

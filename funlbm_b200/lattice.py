@@ -17,7 +17,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import LbmForce, LbmLattice, LbmObserve, call, ptr
+from ._lib import LbmForce, LbmLattice, LbmObserve, addr, call, ptr
 
 BC = {"PERIODICAL": 11000, "WALL": 1200, "WALL_WITH_SPEED": 1201, "NON_EQUILIBRIUM": 1400}
 STORAGE_DTYPE = {"fp32": torch.float32, "fp16s": torch.float16, "bf16s": torch.bfloat16,
@@ -30,29 +30,42 @@ FP16_SCALE = 4096.0
 VECTOR_ELEMS = {"fp32": 4, "fp16s": 8, "bf16s": 8, "fp64": 2}
 
 
-# 16-bit lattices of at least this many nodes pitch rows of odd length
-PITCH_MIN_NODES = 1 << 24
-
-
 def default_pitch(shape, storage):
-    """Whether a lattice pitches its population rows unless told otherwise:
-    16-bit storage, rows of odd length, at least 2^24 nodes.  Measured on
-    B200 (D3Q19 fp16s): pitched rows let node pairs run and win 9 % at 257^3
-    (322 against 351 us per step on dense rows); on the walled 161x65x65
-    and 257x129x129 lattices one node per thread on dense rows wins (23.0
-    against 27.0 us, 162.6 against 173.2 us); in FP32 dense rows win
-    (257^3: 435 us dense, 448 us pitched)."""
-    shape = tuple(int(s) for s in shape)
-    return (BYTES[storage] == 2 and shape[2] % 2 == 1
-            and shape[0] * shape[1] * shape[2] >= PITCH_MIN_NODES)
+    """Whether a lattice pads its population rows unless told otherwise: rows
+    of odd length (the reference's size + 1 nodes for even sizes) in float32
+    or 16-bit storage, by one element, so that the step runs node pairs.
+    Measured on B200, us per step on dense rows (one node per thread) / with
+    rows of nz + 1 elements / with rows of the vector width:
+    257 x 129 x 129 D3Q27 fp32 163 / 150 / 168, fp16s 123 / 96 / 111;
+    177 x 113 x 97 D3Q19 fp32 52.6 / 50.4 / 60.4, fp16s 37.4 / 30.7 / 38.5;
+    129^3 D3Q15 fp32 46.4 / 45.0 / 50.3, fp16s 39.4 / 28.5 / 32.2;
+    257^3 D3Q19 fp32 417 / 402 / -, fp16s 292 / 240 / 259 (281 with 4 nodes per
+    thread); D3Q13 fp16s 223 / 170 / 169."""
+    X, Y, Z = (int(s) for s in shape)
+    return (storage != "fp64" and Z % 2 == 1 and Z >= 3
+            and X * Y * (Z + 1) < 1 << 31)       # (one lattice: under 2^31 elements)
+
+
+def default_pz(shape, storage):
+    """Row pitch of a lattice unless told otherwise."""
+    return int(shape[2]) + (1 if default_pitch(shape, storage) else 0)
 
 
 def row_pitch(nz, storage):
-    """Row pitch of the population buffers: nz rounded up to the widest vector,
-    so that rows of any length (the reference's size + 1 nodes are odd for
-    even sizes) run the vectorised step."""
+    """Row pitch of vector width: nz rounded up to the widest vector, so that
+    rows of any length run every vectorised step."""
     w = VECTOR_ELEMS[storage]
     return -(-int(nz) // w) * w
+
+
+def pitch_of(pitch, shape, storage):
+    """Row pitch in elements for a ``pitch`` argument: None = the default,
+    False = dense rows, True = the vector width, a number = that pitch."""
+    if pitch is None:
+        return default_pz(shape, storage)
+    if pitch is True:
+        return row_pitch(shape[2], storage)
+    return int(pitch) if pitch else int(shape[2])
 
 
 # arithmetic type of a storage: what its fields, face densities, force fields
@@ -100,11 +113,8 @@ class Lattice:
         self.q = int(q)
         self.shape = tuple(int(s) for s in shape)
         self.n = self.shape[0] * self.shape[1] * self.shape[2]
-        # population rows pitched to the vector width (pitch=False: dense
-        # rows; None: default_pitch)
-        if pitch is None:
-            pitch = default_pitch(self.shape, storage)
-        self.pz = row_pitch(self.shape[2], storage) if pitch else self.shape[2]
+        # row pitch of the population buffers (see pitch_of)
+        self.pz = pitch_of(pitch, self.shape, storage)
         self.np = self.shape[0] * self.shape[1] * self.pz
         self.storage = storage
         self.device = torch.device(device)
@@ -148,10 +158,7 @@ class Lattice:
     # -- memory ------------------------------------------------------------
     @staticmethod
     def bytes_needed(q, shape, storage="fp32", pitch=None):
-        if pitch is None:
-            pitch = default_pitch(shape, storage)
-        pz = row_pitch(shape[2], storage) if pitch else int(shape[2])
-        n = int(shape[0]) * int(shape[1]) * pz
+        n = int(shape[0]) * int(shape[1]) * pitch_of(pitch, shape, storage)
         planes = 2 * (shape[1] * shape[2] + shape[0] * shape[2] + shape[0] * shape[1])
         return 2 * q * n * BYTES[storage] + 2 * REAL_DTYPE[storage].itemsize * planes
 
@@ -205,10 +212,10 @@ class Lattice:
 
     def step(self, force=None, obs=None):
         nxt = self.cur ^ 1
-        call("lbm_flow_step", ctypes_ref(self.desc), ptr(self.buf[self.cur]), ptr(self.buf[nxt]),
-             None if force is None else ctypes_ref(force), ptr(self.face_rho[self.cur]),
-             ptr(self.face_rho[nxt]), None if obs is None else ctypes_ref(obs),
-             ptr(self.status), self.stream())
+        call("lbm_flow_step", ctypes_ref(self.desc), addr(self.buf[self.cur]), addr(self.buf[nxt]),
+             None if force is None else ctypes_ref(force), addr(self.face_rho[self.cur]),
+             addr(self.face_rho[nxt]), None if obs is None else ctypes_ref(obs),
+             addr(self.status), self.stream())
         self.cur = nxt
 
     def observe(self, force, f=None, rho=None, u=None):
@@ -252,8 +259,8 @@ class Lattice:
 
 def make_force(old_uniform=(0, 0, 0), new_uniform=(0, 0, 0), old_field=None, new_field=None,
                old_chunks=None, new_chunks=None):
-    return LbmForce(tuple(old_uniform), tuple(new_uniform), ptr(old_field), ptr(new_field),
-                    ptr(old_chunks), ptr(new_chunks))
+    return LbmForce(tuple(old_uniform), tuple(new_uniform), addr(old_field), addr(new_field),
+                    addr(old_chunks), addr(new_chunks))
 
 
 ctypes_ref = ctypes.byref

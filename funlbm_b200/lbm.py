@@ -39,7 +39,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from ._lib import call, ptr
+from ._lib import addr, call, ptr
 from .config import BaseConfig, FileConfig, deep_get
 from .flow import FlowConfig, FlowD3, create_flow
 from .lattice import ctypes_ref, make_force
@@ -476,10 +476,10 @@ class LBMD3(LBMBase):
         sw.ensure_extremes()
         force = make_force(g_old, g_new, *keep)
         cur, nxt = lat.cur, lat.cur ^ 1
-        call("lbm_coupled_step", ctypes_ref(lat.desc), ptr(lat.buf[cur]), ptr(lat.buf[nxt]),
-             ctypes_ref(force), ptr(lat.face_rho[cur]), ptr(lat.face_rho[nxt]),
+        call("lbm_coupled_step", ctypes_ref(lat.desc), addr(lat.buf[cur]), addr(lat.buf[nxt]),
+             ctypes_ref(force), addr(lat.face_rho[cur]), addr(lat.face_rho[nxt]),
              ctypes_ref(sw.struct()), float(cfg.dt), float(cfg.dx), float(cfg.flow_config.gl), 1.0,
-             int(self.step), ptr(self._owner), ptr(self._status_ibm), ptr(lat.status),
+             int(self.step), addr(self._owner), addr(self._status_ibm), addr(lat.status),
              self._stream())
         sw.ext_valid = True
         fl.stepped_elsewhere(force, keep[1], g_new, keep=keep)

@@ -38,7 +38,7 @@ import torch
 
 from . import _lib
 from ._lib import call, ptr
-from .lattice import REAL_DTYPE, Lattice, ctypes_ref
+from .lattice import REAL_DTYPE, Lattice, ctypes_ref, default_pz
 
 _ids = itertools.count()
 
@@ -252,10 +252,10 @@ class LBMServer:
                 flow = r.config.get("flow") or {}
                 q = int(str(flow.get("param_type") or "D3Q19")[3:])
                 storage = ((flow.get("precision") or {}).get("storage")) or "fp32"
-                nz = _shape_of(r.config)[2]
+                pz = default_pz(_shape_of(r.config), storage)
                 forced = bool(r.config.get("particles")) or any(
                     float(v) != 0.0 for v in (flow.get("body_force") or ()))
-                tune_class_of(q, storage, nz, forced, device=self.device)
+                tune_class_of(q, storage, pz, forced, device=self.device)
         torch.cuda.synchronize(self.device)
 
     def _tune(self, lbm):

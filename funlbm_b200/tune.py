@@ -40,13 +40,13 @@ def shape_ok(nodes, pz, bits, nz=None):
     return pz % nodes == 0 and pz >= 2 * nodes
 
 
-def default_shape(q, storage, pz, forced=False):
+def default_shape(q, storage, pz, forced=False, padded=False):
     """The launch shape lbm_flow_step uses when none is set (measured best on
     B200): node pairs with 128 threads where the rows allow them, 4 nodes per
-    thread for unforced D3Q13 / D3Q19 in 16-bit and D3Q15 in bf16s storage,
-    else one node per thread."""
+    thread for unforced D3Q13 in 16-bit, and on rows without padding D3Q19 in
+    16-bit and D3Q15 in bf16s storage, else one node per thread."""
     bits = STORAGE_BITS[storage]
-    four = bits == 16 and (q in (13, 19) or (q == 15 and storage == "bf16s"))
+    four = bits == 16 and (q == 13 or (not padded and (q == 19 or (q == 15 and storage == "bf16s"))))
     want = 4 if four and not forced else 2
     for nodes in (want, 2):
         if pz % nodes == 0 and pz >= 2 * nodes:
@@ -83,7 +83,7 @@ def tune(lat, force=None, iters=6, warmup=2, verbose=False):
     px = max(4, min(nx, PROXY_BYTES // max(per_x, 1)))
     proxy = Lattice(lat.q, (px, ny, nz), lat.faces, lat.tau, storage=lat.storage,
                     face_uw=lat.face_uw, re_mu=lat.re_mu, device=lat.device,
-                    pitch=lat.pz != nz)      # the lattice's own row layout
+                    pitch=lat.pz)            # the lattice's own row layout
     proxy.init(None)
     timings = {}
     start = torch.cuda.Event(enable_timing=True)
@@ -102,7 +102,8 @@ def tune(lat, force=None, iters=6, warmup=2, verbose=False):
         timings[(nodes, threads)] = start.elapsed_time(stop) / iters
     proxy.release()
     del proxy
-    choice = _pick(timings, default_shape(lat.q, lat.storage, lat.pz, force is not None))
+    choice = _pick(timings, default_shape(lat.q, lat.storage, lat.pz, force is not None,
+                                          lat.pz != nz))
     if verbose:
         for k, v in sorted(timings.items(), key=lambda kv: kv[1]):
             print("tune q=%d %s %dx%dx%d (proxy nx=%d): nodes=%d threads=%d  %.4f ms"

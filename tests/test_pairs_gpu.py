@@ -1,0 +1,154 @@
+"""Launch forms against each other, bit for bit: node pairs in packed
+arithmetic against one node per thread, the combined library calls against the
+calls they stand for, fields observed one at a time against all at once."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from tests.gpu_util import init_with, lbm_config, require_cuda, run, smooth_f0
+
+pytestmark = pytest.mark.gpu
+W, P, S = 1200, 11000, 1201
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    require_cuda()
+
+
+def _forced_run(q, storage, shape, faces, pitch, nodes, seed):
+    """Five steps under a body force and random force fields in random 32-node
+    chunks; f, rho and u of the last one."""
+    from funlbm_b200.lattice import Lattice, make_force, tau_float32
+
+    g = torch.Generator().manual_seed(seed)
+    lat = Lattice(q, shape, faces, tau_float32(0.06), storage=storage, pitch=pitch,
+                  face_uw=[(0.01 * i, -0.02, 0.015) for i in range(6)])
+    lat.set_launch_shape(nodes, 128)
+    lat.init(torch.tensor(smooth_f0(q, shape, 0.05, seed)).cuda().permute(3, 0, 1, 2).contiguous()
+             .view(q, -1))
+    fields, flags = [], []
+    for _ in range(2):
+        fl = (torch.rand((lat.n + 31) // 32, generator=g) < 0.4).to(torch.uint8)
+        f = 1e-4 * torch.randn(lat.n, 3, generator=g)
+        f *= (torch.rand(lat.n, 1, generator=g) < 0.5) * fl.repeat_interleave(32)[:lat.n, None]
+        fields.append(f.cuda().reshape(-1))
+        flags.append(fl.cuda())
+    for k in range(5):
+        old, new = k % 2, 1 - k % 2
+        force = make_force((0, 0, 0), (0, 0, 0) if k < 3 else (1e-5, 0, -2e-5), fields[old],
+                           fields[new], flags[old], flags[new])
+        lat.step(force)
+    out = [torch.empty((q, lat.n), device="cuda"), torch.empty(lat.n, device="cuda"),
+           torch.empty((lat.n, 3), device="cuda")]
+    lat.observe(force, *out)
+    for k in range(3):       # each of them alone
+        one = [None, None, None]
+        one[k] = torch.empty_like(out[k])
+        lat.observe(force, *one)
+        assert torch.equal(one[k], out[k]), k
+    assert lat.read_status() == 0
+    return [t.cpu().numpy() for t in out]
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s", "bf16s"])
+@pytest.mark.parametrize("q", [13, 15, 19, 27])
+@pytest.mark.parametrize("shape,faces", [
+    ((6, 5, 33), [W, P, P, W, S, W]),      # rows padded by one, a partial last pair
+    ((5, 9, 35), [S, W, W, S, P, P]),
+    ((4, 7, 5), [P] * 6),                  # a row of three pairs
+    ((5, 6, 32), [P, P, S, W, W, S]),      # even rows, no padding
+])
+def test_pairs_equal_single_nodes(q, storage, shape, faces):
+    dense = _forced_run(q, storage, shape, faces, False, 1, 3)
+    forms = [(None, 2), (True, 2)]
+    if storage != "fp32" or shape[2] > 8:
+        forms.append((True, 4))
+    for pitch, nodes in forms:
+        got = _forced_run(q, storage, shape, faces, pitch, nodes, 3)
+        for a, b in zip(dense, got):
+            assert np.array_equal(a, b), (pitch, nodes)
+
+
+@pytest.mark.parametrize("q", [13, 19, 27])
+@pytest.mark.parametrize("faces", [[1400, 1400, W, W, W, W], [1400, W, P, P, W, S], [W, P, S, W, P, P]])
+def test_compute_flow_equals_its_calls(q, faces):
+    from funlbm_b200.lbm import LBMD3
+
+    def flow():
+        lbm = LBMD3(config=lbm_config(q, (9, 6, 11), 0.1, faces,
+                                      uw=[(0.01, 0.02, -0.01)] * 6, fused=False))
+        init_with(lbm, smooth_f0(q, (10, 7, 12), 0.03, 5))
+        lbm.flow.FOL = 1e-5 * torch.randn((10, 7, 12, 3), generator=torch.Generator().manual_seed(1))
+        return lbm.flow
+
+    a, b = flow(), flow()
+    for _ in range(3):
+        a.compute_flow()
+        b.cul_equ()
+        b.f_stream()
+        b.update_u_rou()
+        for k in ("f", "rou", "u", "p", "feq"):
+            assert torch.equal(getattr(a, k), getattr(b, k)), k
+
+
+def test_no_force_step_skips_nothing_that_counts():
+    """Non-equilibrium channel: steps that skip the forcing pass against steps
+    that run it on a FOL of zeros, and a replaced method is still called."""
+    from funlbm_b200.lbm import LBMD3
+
+    def make():
+        lbm = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+        init_with(lbm, smooth_f0(19, (10, 7, 8), 0.02, 2))
+        return lbm
+
+    a, b, c = make(), make(), make()
+    calls = []
+    plain = b.lagrange_to_flow
+    b.lagrange_to_flow = lambda *args: (calls.append(1), plain(*args))
+    c.flow.FOL = 1e-4 * torch.ones((10, 7, 8, 3))       # dropped by the first step's spreading
+    for lbm in (a, b, c):
+        run(lbm, 4)
+    assert len(calls) == 4
+    for k in ("f", "rou", "u"):
+        assert torch.equal(getattr(a.flow, k), getattr(b.flow, k)), k
+    assert float(c.flow.FOL.abs().max()) == 0.0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s", "fp64"])
+def test_coupled_step_equals_its_calls(storage):
+    from funlbm_b200.lbm import LBMD3
+
+    parts = [{"type": "sphere", "r": 3, "rou": 1.3, "coord": {"center": [12, 9, 9]}},
+             {"type": "ellipsoid", "a": 4, "b": 2, "c": 2, "rou": 1.1,
+              "coord": {"center": [18, 8, 10], "alpha": 0.3, "beta": 0.5, "gamma": 0.1}}]
+
+    def make():
+        lbm = LBMD3(config=lbm_config(19, (24, 18, 20), 0.08, [W, W, P, P, W, W], gl=1e-3,
+                                      storage=storage, particles=parts, body_force=(0, 1e-6, 0)))
+        lbm.init()
+        return lbm
+
+    a, b = make(), make()
+    b._coupled_step = lambda: False
+    for lbm in (a, b):
+        run(lbm, 7)
+    for k in ("f", "u", "rou", "FOL"):
+        assert torch.equal(getattr(a.flow, k), getattr(b.flow, k)), k
+    for k in ("lx", "lF", "cx", "cu", "cw", "angle", "extreme"):
+        assert torch.equal(getattr(a.particle_swarm, k), getattr(b.particle_swarm, k)), k
+
+
+def test_coupled_step_refuses_what_it_needs():
+    from funlbm_b200 import _lib
+    from funlbm_b200.lattice import Lattice, make_force
+
+    lat = Lattice(19, (8, 8, 8), [W] * 6, 0.7)
+    pt = _lib.LbmParticles()
+    pt.n_particles, pt.n_markers = 1, 1
+    with pytest.raises(ValueError):
+        _lib.call("lbm_coupled_step", ctypes.byref(lat.desc), lat.buf[0].data_ptr(),
+                  lat.buf[1].data_ptr(), ctypes.byref(make_force()), None, None, ctypes.byref(pt),
+                  1.0, 1.0, 0.0, 1.0, 1, None, None, None, lat.stream())
