@@ -117,7 +117,8 @@ SIGNATURES = {
     "lbm_stream": (I, [_LAT, _P, _P, _P, _P, _P]),
     "lbm_moments": (I, [_LAT, _P, _P, _P, _P, _P, _P, _P]),
     "lbm_coupled_step": (I, [_LAT, _P, _P, _FORCE, _P, _P, _PART, F, F, F, F, ctypes.c_int32, _P,
-                             _P, _P, _P]),
+                             _P, ctypes.c_size_t, ctypes.c_int32, _P, _P, _P]),
+    "lbm_coupled_scratch_bytes": (ctypes.c_size_t, [_LAT, ctypes.c_int32, ctypes.c_int32]),
     "lbm_compute_flow": (I, [_LAT, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "lbm_add_force": (I, [_LAT, _P, _P, _P, _P]),
     "ibm_interpolate": (I, [_LAT, _P, _FORCE, _P, _P, _P, _PART, F, ctypes.c_int32, _P, _P]),

@@ -53,14 +53,8 @@ __device__ __forceinline__ unsigned bad_bits(R rho, R ux, R uy, R uz) {
   return b;
 }
 
-// Everything after the pull for one node: the previous / new forcing, the
-// moment passes, cul_equ2, status bits (accumulated in `bad`), face
-// densities, observation, and (when fb is set) the next step's collision, in
-// place in f.  DEV: f holds deviations d = f - w (shifted storage), handled
-// by dev_moments / collide_dev.
 // Whether the previous / this step's force field applies in the 32-node
-// chunk of node idx.  A thread's nodes always share one chunk, so the kernels
-// read the flags once, before their population loads.
+// chunk of node idx.
 struct ChunkForce {
   bool old_here, new_here;
 };
@@ -89,8 +83,12 @@ __device__ __forceinline__ void node_force(const float uniform[3], const void *f
   }
 }
 
-// finish_node_m hands the node's end-of-step moments (the second
-// update_u_rou) to the caller; f is left at the end-of-step populations.
+// Everything after the pull for one node: the first moments with the previous
+// force, cul_equ2 with the new one, the second moments, status bits
+// (accumulated in `bad`) and face densities.  DEV: f holds deviations d = f - w
+// (shifted storage), handled by dev_moments / collide_dev.  finish_node_m hands
+// the node's end-of-step moments to the caller; f is left at the end-of-step
+// populations.
 // Where neither step has a force (no uniform part, neither field in the
 // node's chunk) cul_equ2 adds nothing and the second moment pass repeats the
 // first, so both are skipped -- the same rule in every kernel, and a node of a

@@ -441,6 +441,7 @@ class LBMD3(LBMBase):
         else:
             # claim array of the global-claim spreading, -1 between calls
             self._owner = torch.full((n,), -1, dtype=torch.int32, device=dev)
+        self._boxes = self._make_boxes()
         self._fi = 0          # index of the buffer the next spread writes
         self._status_ibm = torch.zeros(1, dtype=torch.int32, device=dev)
         # FOL of the state being entered (zero after init): the next step's
@@ -457,6 +458,35 @@ class LBMD3(LBMBase):
         plan = self.fused_prepare()
         self.flow.fused_step(plan["force"], plan["new_field"], plan["g_new"], keep=plan["keep"])
         self.fused_finish(plan)
+
+    # Markers from which the moments around the particles are taken once per
+    # node (lbm_coupled_step's scratch): below, the extra launch costs what it
+    # saves (us per step without / with: 1,160 markers 36.8 / 41.2, 2,600
+    # markers 58.4 / 59.1, 11,776 markers 226 / 202)
+    _BOX_MARKERS = 5000
+    _BOX_BYTES = 256 << 20
+
+    def _make_boxes(self):
+        """lbm_coupled_step's scratch, allocated with the IBM buffers: (buffer,
+        cells per particle, particles), or None when there are few markers or
+        the boxes would be too large."""
+        sw = self.particle_swarm
+        count = len(sw.particles)
+        if not count or sw.n_markers < max(1, self._BOX_MARKERS):
+            return None
+        # a box holds every rotation of the largest body and its stencils
+        cells = int(2 * float(sw.lagrange.norm(dim=1).max()) + 7) ** 3
+        if cells > 1 << 24:
+            return None
+        nb = _lib.load().lbm_coupled_scratch_bytes(ctypes_ref(self.flow.lattice.desc), count, cells)
+        if nb > self._BOX_BYTES:
+            return None
+        return torch.empty(nb, dtype=torch.uint8, device=self.device), cells, count
+
+    def _box_scratch(self):
+        if self._boxes is None or self._boxes[2] != len(self.particle_swarm.particles):
+            return None, 0, 0
+        return self._boxes[0].data_ptr(), self._boxes[0].numel(), self._boxes[1]
 
     def _coupled_step(self):
         """A step with particles and claimed spreading in one library call
@@ -479,8 +509,8 @@ class LBMD3(LBMBase):
         call("lbm_coupled_step", ctypes_ref(lat.desc), addr(lat.buf[cur]), addr(lat.buf[nxt]),
              ctypes_ref(force), addr(lat.face_rho[cur]), addr(lat.face_rho[nxt]),
              ctypes_ref(sw.struct()), float(cfg.dt), float(cfg.dx), float(cfg.flow_config.gl), 1.0,
-             int(self.step), addr(self._owner), addr(self._status_ibm), addr(lat.status),
-             self._stream())
+             int(self.step), addr(self._owner), *self._box_scratch(), addr(self._status_ibm),
+             addr(lat.status), self._stream())
         sw.ext_valid = True
         fl.stepped_elsewhere(force, keep[1], g_new, keep=keep)
         self._fi = old

@@ -356,15 +356,22 @@ int ibm_spread_claimed(const lbm_lattice *lat, const lbm_particles *pt, float *f
  * Same results as the two calls. */
 int rigid_step(const lbm_particles *pt, float dt, float gl, float rouf, void *stream);
 
+/* Bytes of lbm_coupled_step's scratch for `cells` nodes per particle box. */
+size_t lbm_coupled_scratch_bytes(const lbm_lattice *lat, int32_t n_particles, int32_t cells);
 /* One fused step of a lattice with particles in one call: the launches of
  * ibm_interpolate_wall_claim (old force of `force`), ibm_spread_claimed into
  * force->new_field / new_chunks, rigid_step and lbm_flow_step, in that order
  * on one stream.  ibm_status: status word of the interpolation; owner: claim
- * array, -1 between calls.  With no particles only the flow step is launched. */
+ * array, -1 between calls.  scratch (may be NULL; 16-byte aligned, contents
+ * undefined between calls): room for the moments of up to `cells` nodes around
+ * each particle, taken once per node instead of once per stencil slot (pays
+ * from a few thousand markers); same results.  With no particles only the flow
+ * step is launched. */
 int lbm_coupled_step(const lbm_lattice *lat, const void *fa, void *fb, const lbm_force *force,
                      const float *face_rho_in, float *face_rho_out, const lbm_particles *pt,
                      float dt, float dx, float gl, float rouf, int32_t step, int32_t *owner,
-                     uint32_t *ibm_status, uint32_t *status, void *stream);
+                     void *scratch, size_t scratch_bytes, int32_t cells, uint32_t *ibm_status,
+                     uint32_t *status, void *stream);
 
 /* The six extreme markers of the current positions into pt->extreme
  * (the argmin / argmax of lbm/lbm3d.py:121-167). */

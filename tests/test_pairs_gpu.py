@@ -141,6 +141,42 @@ def test_coupled_step_equals_its_calls(storage):
         assert torch.equal(getattr(a.particle_swarm, k), getattr(b.particle_swarm, k)), k
 
 
+@pytest.mark.parametrize("storage", ["fp32", "bf16s", "fp64"])
+@pytest.mark.parametrize("cells", [None, 900, 60])
+def test_box_moments_equal_slot_moments(storage, cells):
+    """Interpolation from moments taken once per node: bodies of two sizes, one
+    across a wall, boxes that do not fit (60: none does, 900: the small
+    body's only)."""
+    from funlbm_b200.lbm import LBMD3
+
+    parts = [{"type": "sphere", "r": 4, "rou": 1.3, "coord": {"center": [12, 9, 9]}},
+             {"type": "sphere", "r": 2, "rou": 1.3, "coord": {"center": [4, 12, 16]}},
+             {"type": "ellipsoid", "a": 4, "b": 3, "c": 2, "rou": 0.9,
+              "coord": {"center": [23, 16, 2], "alpha": 0.3, "beta": 0.5, "gamma": 0.1}}]
+
+    def make(least):
+        lbm = LBMD3(config=lbm_config(19, (25, 19, 20), 0.08, [W, W, P, P, W, S], gl=1e-3,
+                                      uw=[(0.0, 0.01, 0.0)] * 6, storage=storage, particles=parts))
+        lbm._BOX_MARKERS = least
+        lbm.init()
+        return lbm
+
+    a, b = make(1), make(10 ** 9)
+    for k in range(8):
+        if k == 2 and cells is not None:
+            a._boxes = (a._boxes[0], cells, 3)
+        if k == 5:          # positions moved in place: the extremes are stale
+            for lbm in (a, b):
+                lbm.particle_swarm.lx[:40] += 5.0
+        for lbm in (a, b):
+            run(lbm, 1)
+    assert a._boxes is not None and b._boxes is None
+    for k in ("f", "u", "rou", "FOL"):
+        assert torch.equal(getattr(a.flow, k), getattr(b.flow, k)), k
+    for k in ("lx", "lF", "lu", "lrou", "cx", "cu", "cw"):
+        assert torch.equal(getattr(a.particle_swarm, k), getattr(b.particle_swarm, k)), k
+
+
 def test_coupled_step_refuses_what_it_needs():
     from funlbm_b200 import _lib
     from funlbm_b200.lattice import Lattice, make_force
@@ -151,4 +187,4 @@ def test_coupled_step_refuses_what_it_needs():
     with pytest.raises(ValueError):
         _lib.call("lbm_coupled_step", ctypes.byref(lat.desc), lat.buf[0].data_ptr(),
                   lat.buf[1].data_ptr(), ctypes.byref(make_force()), None, None, ctypes.byref(pt),
-                  1.0, 1.0, 0.0, 1.0, 1, None, None, None, lat.stream())
+                  1.0, 1.0, 0.0, 1.0, 1, None, None, 0, 0, None, None, lat.stream())
