@@ -466,6 +466,19 @@ class LBMD3(LBMBase):
     _BOX_MARKERS = 5000
     _BOX_BYTES = 256 << 20
 
+    @staticmethod
+    def _box_cells(lagrange, count):
+        """Cells of a box that holds every rotation of the largest body and its
+        stencils; 0 when the boxes of `count` particles together hold more
+        nodes than the 64 stencil slots of each marker (few small bodies
+        beside a large one, markers far apart: a pass over the boxes would
+        cost more than the pulls it saves) or a marker is not finite."""
+        side = 2 * float(lagrange.norm(dim=1).max()) + 7
+        if not side < 257:
+            return 0
+        cells = int(side) ** 3
+        return cells if count * cells <= 64 * lagrange.shape[0] else 0
+
     def _make_boxes(self):
         """lbm_coupled_step's scratch, allocated with the IBM buffers: (buffer,
         cells per particle, particles), or None when there are few markers or
@@ -474,12 +487,9 @@ class LBMD3(LBMBase):
         count = len(sw.particles)
         if not count or sw.n_markers < max(1, self._BOX_MARKERS):
             return None
-        # a box holds every rotation of the largest body and its stencils
-        cells = int(2 * float(sw.lagrange.norm(dim=1).max()) + 7) ** 3
-        if cells > 1 << 24:
-            return None
+        cells = self._box_cells(sw.lagrange, count)
         nb = _lib.load().lbm_coupled_scratch_bytes(ctypes_ref(self.flow.lattice.desc), count, cells)
-        if nb > self._BOX_BYTES:
+        if cells == 0 or nb > self._BOX_BYTES:
             return None
         return torch.empty(nb, dtype=torch.uint8, device=self.device), cells, count
 
