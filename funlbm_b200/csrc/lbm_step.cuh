@@ -337,6 +337,7 @@ __global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q
 template <int Q, int S, bool FORCE>
 __global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q, S>()))
     k_observe(const __grid_constant__ StepArgs a) {
+  chain_enter();
   step_scalar_body<Q, S, FORCE, Op::kObserve>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
 }
 
@@ -818,6 +819,7 @@ __global__ void __launch_bounds__(TB, (vec_min_blocks<Q, S, NZ, TB, FORCE>()))
 // The end-of-step state to the observation buffers, two nodes per thread.
 template <int Q, int S, bool FORCE, bool PITCH>
 __global__ void __launch_bounds__(128) k_observe_vec(const __grid_constant__ StepArgs a) {
+  chain_enter();
   step_pairs_at<Q, S, FORCE, 2, PITCH, Op::kObserve>(a, 2u * (blockIdx.x * 128u + threadIdx.x));
 }
 
