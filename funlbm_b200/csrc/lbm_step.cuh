@@ -142,10 +142,46 @@ __device__ __forceinline__ void observe_node(const StepArgs &a, const R f[Q], un
   }
 }
 
-// What a launch does with its nodes: advance them (collide and store) or
-// write their end-of-step state (a kernel of its own, so the step carries
-// none of that code).
-enum class Op { kStep, kObserve };
+// The same for nodes idx and (two) idx + 1, as aligned stores of both where the
+// buffers allow them.
+template <int Q, int SH>
+__device__ __forceinline__ void observe_pair(const StepArgs &a, const F2 f[Q], unsigned idx,
+                                             bool two, F2 rho, F2 ux, F2 uy, F2 uz) {
+  if (!two || !a.obs_pairs) {
+    float fa[Q], fb[Q];
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      fa[i] = f[i].v.x;
+      fb[i] = f[i].v.y;
+    });
+    observe_node<Q, true, SH>(a, fa, idx, rho.v.x, ux.v.x, uy.v.x, uz.v.x);
+    if (two) observe_node<Q, true, SH>(a, fb, idx + 1, rho.v.y, ux.v.y, uy.v.y, uz.v.y);
+    return;
+  }
+  if (a.obs_f != nullptr) {
+    float *of = static_cast<float *>(a.obs_f);
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      const F2 v = f[i] * F2(1.f / (float)(1 << SH)) + F2(VSet<Q>::w(i));
+      *reinterpret_cast<float2 *>(of + (long long)i * a.g.n + idx) = v.v;
+    });
+  }
+  if (a.obs_rho != nullptr)
+    *reinterpret_cast<float2 *>(static_cast<float *>(a.obs_rho) + idx) = rho.v;
+  if (a.obs_u != nullptr) {
+    float2 *ou = reinterpret_cast<float2 *>(static_cast<float *>(a.obs_u) + 3ull * idx);
+    ou[0] = make_float2(ux.v.x, uy.v.x);
+    ou[1] = make_float2(uz.v.x, ux.v.y);
+    ou[2] = make_float2(uy.v.y, uz.v.y);
+  }
+}
+
+// What a launch does with its nodes: advance them (collide and store), write
+// their end-of-step state, or both in one read of the populations (kernels of
+// their own, so the step carries none of that code).
+enum class Op { kStep, kObserve, kBoth };
+__host__ __device__ constexpr bool advances(Op op) { return op != Op::kObserve; }
+__host__ __device__ constexpr bool observes(Op op) { return op != Op::kStep; }
 
 template <int Q, bool FORCE, bool DEV, int SH, Op OP, typename R>
 __device__ __forceinline__ void finish_node(const StepArgs &a, R f[Q], unsigned idx, int x,
@@ -153,12 +189,13 @@ __device__ __forceinline__ void finish_node(const StepArgs &a, R f[Q], unsigned 
                                             unsigned &bad) {
   R rho, drho, ux, uy, uz;
   finish_node_m<Q, FORCE, DEV, SH>(a, f, idx, x, y, z, face, cf, bad, rho, drho, ux, uy, uz);
-  if constexpr (OP == Op::kObserve)
-    observe_node<Q, DEV, SH>(a, f, idx, rho, ux, uy, uz);
-  else if constexpr (DEV)
-    collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
-  else
-    collide<Q>(f, a.g, rho, ux, uy, uz);
+  if constexpr (observes(OP)) observe_node<Q, DEV, SH>(a, f, idx, rho, ux, uy, uz);
+  if constexpr (advances(OP)) {
+    if constexpr (DEV)
+      collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
+    else
+      collide<Q>(f, a.g, rho, ux, uy, uz);
+  }
 }
 
 // finish_node for two neighbouring nodes (z, z + 1) of a row at once, in
@@ -197,37 +234,8 @@ __device__ __forceinline__ void finish_pair(const StepArgs &a, F2 f[Q], unsigned
     if (face.a) write_face_rho<Q>(a.g, fr, x, y, z, rho.v.x);
     if (face.b && two) write_face_rho<Q>(a.g, fr, x, y, z + 1, rho.v.y);
   }
-  if constexpr (OP == Op::kStep) {
-    collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
-  } else {
-    if (!two || !a.obs_pairs) {
-      float fa[Q], fb[Q];
-      static_for<Q>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        fa[i] = f[i].v.x;
-        fb[i] = f[i].v.y;
-      });
-      observe_node<Q, true, SH>(a, fa, idx, rho.v.x, ux.v.x, uy.v.x, uz.v.x);
-      if (two) observe_node<Q, true, SH>(a, fb, idx + 1, rho.v.y, ux.v.y, uy.v.y, uz.v.y);
-      return;
-    }
-    if (a.obs_f != nullptr) {
-      float *of = static_cast<float *>(a.obs_f);
-      static_for<Q>([&](auto ic) {
-        constexpr int i = decltype(ic)::value;
-        const F2 v = f[i] * F2(1.f / (float)(1 << SH)) + F2(VSet<Q>::w(i));
-        *reinterpret_cast<float2 *>(of + (long long)i * a.g.n + idx) = v.v;
-      });
-    }
-    if (a.obs_rho != nullptr)
-      *reinterpret_cast<float2 *>(static_cast<float *>(a.obs_rho) + idx) = rho.v;
-    if (a.obs_u != nullptr) {
-      float2 *ou = reinterpret_cast<float2 *>(static_cast<float *>(a.obs_u) + 3ull * idx);
-      ou[0] = make_float2(ux.v.x, uy.v.x);
-      ou[1] = make_float2(uz.v.x, ux.v.y);
-      ou[2] = make_float2(uy.v.y, uz.v.y);
-    }
-  }
+  if constexpr (observes(OP)) observe_pair<Q, SH>(a, f, idx, two, rho, ux, uy, uz);
+  if constexpr (advances(OP)) collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
 }
 
 __device__ __forceinline__ void report_bad(unsigned *status, unsigned bad) {
@@ -294,7 +302,7 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
   finish_node<Q, FORCE, St::kDev, St::kShift, OP>(a, f, idx, x, y, z, on_any_face(a.g, x, y, z), cf,
                                                   bad);
   report_bad(a.status, bad);
-  if constexpr (OP == Op::kStep) {
+  if constexpr (advances(OP)) {
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       St::put(static_cast<T *>(a.p.dst[i]) + pidx, f[i]);
@@ -332,13 +340,13 @@ __global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q
   step_scalar_body<Q, S, FORCE>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
 }
 
-// The end-of-step state of every node to the observation buffers, nothing
-// stored back: one node per thread (rows that take no pairs, FP64).
-template <int Q, int S, bool FORCE>
+// The end-of-step state of every node to the observation buffers, and with
+// Op::kBoth the step itself: one node per thread (rows that take no pairs, FP64).
+template <int Q, int S, bool FORCE, Op OP>
 __global__ void __launch_bounds__((scalar_threads<Q, S>()), (scalar_min_blocks<Q, S>()))
     k_observe(const __grid_constant__ StepArgs a) {
   chain_enter();
-  step_scalar_body<Q, S, FORCE, Op::kObserve>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
+  step_scalar_body<Q, S, FORCE, OP>(a, blockIdx.x * scalar_threads<Q, S>() + threadIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -568,7 +576,7 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
   a.pdec(pidx0, x, y, z0);
   if constexpr (PITCH) {
     if (z0 >= a.g.nz) {                      // row padding only
-      if constexpr (OP == Op::kStep) put_padding_vector<Q, S, NZ>(a, pidx0);
+      if constexpr (advances(OP)) put_padding_vector<Q, S, NZ>(a, pidx0);
       return;
     }
   }
@@ -638,7 +646,7 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
   if constexpr (FORCE) {
     if (((idx0 + nv - 1) >> 5) != (idx0 >> 5)) cf1 = chunk_force<FORCE>(a, idx0 + nv - 1);
   }
-  Words<kWords> out[OP == Op::kStep ? Q : 1];
+  Words<kWords> out[advances(OP) ? Q : 1];
 #pragma unroll
   for (int pr = 0; pr < NZ / 2; ++pr) {
     const int k0 = 2 * pr, k1 = 2 * pr + 1;
@@ -693,7 +701,7 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
                                             !PITCH || k1 < nv, s0 ? cf0 : cf1, s1 ? cf0 : cf1,
                                             bad);
     }
-    if constexpr (OP == Op::kStep) {
+    if constexpr (advances(OP)) {
       static_for<Q>([&](auto ic) {
         constexpr int i = decltype(ic)::value;
         if constexpr (St::kBits == 32) {
@@ -706,7 +714,7 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
     }
   }
   report_bad(a.status, bad);
-  if constexpr (OP == Op::kStep) {
+  if constexpr (advances(OP)) {
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
       T *dst = static_cast<T *>(a.p.dst[i]) + pidx0;
@@ -816,11 +824,11 @@ __global__ void __launch_bounds__(TB, (vec_min_blocks<Q, S, NZ, TB, FORCE>()))
   step_vec_body<Q, S, FORCE, NZ, PITCH>(a, blockIdx.x * TB + threadIdx.x);
 }
 
-// The end-of-step state to the observation buffers, two nodes per thread.
-template <int Q, int S, bool FORCE, bool PITCH>
+// The same, two nodes per thread.
+template <int Q, int S, bool FORCE, bool PITCH, Op OP>
 __global__ void __launch_bounds__(128) k_observe_vec(const __grid_constant__ StepArgs a) {
   chain_enter();
-  step_pairs_at<Q, S, FORCE, 2, PITCH, Op::kObserve>(a, 2u * (blockIdx.x * 128u + threadIdx.x));
+  step_pairs_at<Q, S, FORCE, 2, PITCH, OP>(a, 2u * (blockIdx.x * 128u + threadIdx.x));
 }
 
 // Rows of odd length in 16-bit storage: thread k of a row takes the node pair
@@ -1224,7 +1232,24 @@ struct StepLauncher {
     else
       force ? go_odd_f<true, 128>(a, s) : go_odd_f<false, 128>(a, s);
   }
-  // Observation launch: two nodes per thread where the rows allow pairs.
+  // Observation launch (Op::kBoth: with the step): two nodes per thread where
+  // the rows allow pairs, whatever the step's own launch shape.
+  template <Op OP, bool FORCE>
+  static void go_observe_f(const StepArgs &a, bool pairs, cudaStream_t s) {
+    if constexpr (Storage<S>::kBits != 64) {
+      if (pairs) {
+        const unsigned nb = blocks_for(a.g.np / 2, 128);
+        if (a.g.pz != a.g.nz)
+          launch_chained(k_observe_vec<Q, S, FORCE, true, OP>, nb, 128, 0, s, a);
+        else
+          launch_chained(k_observe_vec<Q, S, FORCE, false, OP>, nb, 128, 0, s, a);
+        return;
+      }
+    }
+    constexpr int tb = scalar_threads<Q, S>();
+    launch_chained(k_observe<Q, S, FORCE, OP>, blocks_for(a.g.n, tb), tb, 0, s, a);
+  }
+  template <Op OP>
   static int go_observe(StepArgs a, bool force, int nodes, cudaStream_t s) {
     constexpr int bits = Storage<S>::kBits;
     if (nodes == LBM_STEP_ROWS) {   // (a lattice that cannot be row-staged is refused here too)
@@ -1236,37 +1261,18 @@ struct StepLauncher {
     }
     const uintptr_t at = (uintptr_t)a.obs_f | (uintptr_t)a.obs_rho | (uintptr_t)a.obs_u;
     a.obs_pairs = a.g.n % 2 == 0 && a.g.nz % 2 == 0 && at % 8 == 0;
-    if constexpr (bits != 64) {
-      if (nodes != 1 && step_shape_ok(2, a.g.pz, bits)) {
-        const unsigned nb = blocks_for(a.g.np / 2, 128);
-        const bool pitch = a.g.pz != a.g.nz;
-        if (force)
-          pitch ? launch_chained(k_observe_vec<Q, S, true, true>, nb, 128, 0, s, a)
-                : launch_chained(k_observe_vec<Q, S, true, false>, nb, 128, 0, s, a);
-        else
-          pitch ? launch_chained(k_observe_vec<Q, S, false, true>, nb, 128, 0, s, a)
-                : launch_chained(k_observe_vec<Q, S, false, false>, nb, 128, 0, s, a);
-        return LBM_OK;
-      }
-    }
-    constexpr int tb = scalar_threads<Q, S>();
-    const unsigned nb = blocks_for(a.g.n, tb);
+    const bool pairs = nodes != 1 && step_shape_ok(2, a.g.pz, bits);
     if (force)
-      launch_chained(k_observe<Q, S, true>, nb, tb, 0, s, a);
+      go_observe_f<OP, true>(a, pairs, s);
     else
-      launch_chained(k_observe<Q, S, false>, nb, tb, 0, s, a);
+      go_observe_f<OP, false>(a, pairs, s);
     return LBM_OK;
   }
   static int go(const StepArgs &a, bool force, int nodes, int threads, cudaStream_t s) {
     constexpr int bits = Storage<S>::kBits;
-    if (a.fb == nullptr) return go_observe(a, force, nodes, s);
-    if (a.obs_f != nullptr || a.obs_rho != nullptr || a.obs_u != nullptr) {
-      StepArgs o = a;   // (the step below reports the status and the face densities)
-      o.status = nullptr;
-      o.face_rho_out = nullptr;
-      const int rc = go_observe(o, force, nodes, s);
-      if (rc) return rc;
-    }
+    if (a.fb == nullptr) return go_observe<Op::kObserve>(a, force, nodes, s);
+    if (a.obs_f != nullptr || a.obs_rho != nullptr || a.obs_u != nullptr)
+      return go_observe<Op::kBoth>(a, force, nodes, s);
     if (nodes == LBM_STEP_ROWS) return go_tma(a, force, s);
     const bool odd_pairs = bits == 16 && a.g.pz % 2 == 1 && a.g.nz >= 3;
     if (nodes == 0) {

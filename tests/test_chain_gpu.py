@@ -92,3 +92,59 @@ def test_steps_around_a_read_stay_in_order():
 
     for a, b in zip(run(True), run(False)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s", "bf16s", "fp64"])
+@pytest.mark.parametrize("nz,pitch,nodes", [
+    (33, None, 0), (33, False, 0), (33, False, 1), (32, None, 0), (32, None, -1), (32, True, 2),
+])
+def test_observed_step_is_one_launch(storage, nz, pitch, nodes):
+    """A step with observation buffers reads the populations once and gives
+    what the step and the observation give apart."""
+    runtime = pytest.importorskip("cuda.bindings.runtime")
+    from funlbm_b200._lib import LbmObserve, ptr
+    from funlbm_b200.lattice import Lattice, make_force, tau_float32
+
+    if storage == "fp64" and nodes == -1:
+        pytest.skip("row staging is not built for FP64")
+    S = 1201
+    shape = (9, 7, nz)
+    lat = Lattice(19, shape, [W, S, P, P, W, S], tau_float32(0.05), storage=storage, pitch=pitch,
+                  face_uw=[(0.01, -0.02, 0.015)] * 6)
+    lat.set_launch_shape(nodes, 128)
+    dt = lat.real_dtype
+    lat.init(torch.tensor(smooth_f0(19, shape, 0.05, 2)).cuda().permute(3, 0, 1, 2)
+             .reshape(19, -1).to(dt).contiguous())
+    force = make_force((1e-5, 0, 0), (0, 2e-5, 0))
+    lat.step(force)
+
+    def fields():
+        return [torch.zeros(s, dtype=dt, device="cuda") for s in ((19, lat.n), (lat.n,), (lat.n, 3))]
+
+    def stored(b):
+        return b.view(19, -1, lat.pz)[:, :, :nz].clone()
+
+    lat.step(force)                                   # apart
+    apart = fields()
+    lat.observe(force, *apart)
+    after, rho_after = stored(lat.buf[lat.cur]), lat.face_rho[lat.cur].clone()
+    lat.cur ^= 1
+    lat.buf[lat.cur ^ 1].zero_()
+    lat.face_rho[lat.cur ^ 1].zero_()
+    both = fields()
+    g = torch.cuda.CUDAGraph(keep_graph=True)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        g.capture_begin()
+        lat.step(force, obs=LbmObserve(*(ptr(t) for t in both)))
+        g.capture_end()
+    err, _, count = runtime.cudaGraphGetNodes(runtime.cudaGraph_t(init_value=g.raw_cuda_graph()), 0)[:3]
+    assert int(err) == 0 and count == 1
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    for a, b in zip(apart, both):
+        assert torch.equal(a, b)
+    assert torch.equal(after, stored(lat.buf[lat.cur]))
+    assert torch.equal(rho_after, lat.face_rho[lat.cur])
+    assert lat.read_status() == 0
