@@ -142,38 +142,84 @@ __device__ __forceinline__ void observe_node(const StepArgs &a, const R f[Q], un
   }
 }
 
-// The same for nodes idx and (two) idx + 1, as aligned stores of both where the
-// buffers allow them.
+// A thread's one or (two) two values into an array that the threads of a warp
+// fill one after the other, in aligned stores of two: where the thread's place
+// is odd, its last value leaves with its right neighbour's first.  lanes: the
+// warp's threads that take part.
+__device__ __forceinline__ void store_run(float *dst, float a, float b, bool two, unsigned lanes) {
+  const unsigned lane = threadIdx.x & 31u;
+  const bool prev = lane > 0u && ((lanes >> (lane - 1u)) & 1u);
+  const bool next = lane < 31u && ((lanes >> (lane + 1u)) & 1u);
+  const float na = __shfl_down_sync(lanes, a, 1);
+  const bool odd = ((uintptr_t)dst & 4u) != 0;
+  if (odd && !prev) dst[0] = a;
+  if (odd && !two) return;
+  const bool own = !odd && two;
+  const float v0 = odd ? b : a, v1 = own ? b : na;
+  dst += odd ? 1 : 0;
+  if (own || next)
+    *reinterpret_cast<float2 *>(dst) = make_float2(v0, v1);
+  else
+    dst[0] = v0;
+}
+// The same for three values a node.
+__device__ __forceinline__ void store_run3(float *dst, F2 vx, F2 vy, F2 vz, bool two,
+                                           unsigned lanes) {
+  const unsigned lane = threadIdx.x & 31u;
+  const bool prev = lane > 0u && ((lanes >> (lane - 1u)) & 1u);
+  const bool next = lane < 31u && ((lanes >> (lane + 1u)) & 1u);
+  const float nx = __shfl_down_sync(lanes, vx.v.x, 1);
+  const bool odd = ((uintptr_t)dst & 4u) != 0;
+  if (odd && !prev) dst[0] = vx.v.x;
+  float2 *d = reinterpret_cast<float2 *>(dst + (odd ? 1 : 0));
+  d[0] = odd ? make_float2(vy.v.x, vz.v.x) : make_float2(vx.v.x, vy.v.x);
+  if (two) d[1] = odd ? make_float2(vx.v.y, vy.v.y) : make_float2(vz.v.x, vx.v.y);
+  if (odd && !two) return;
+  const float v0 = two ? (odd ? vz.v.y : vy.v.y) : vz.v.x;
+  const float v1 = two && !odd ? vz.v.y : nx;
+  if (two) ++d;
+  if ((two && !odd) || next)
+    d[1] = make_float2(v0, v1);
+  else
+    *reinterpret_cast<float *>(d + 1) = v0;
+}
+
+// The same for nodes idx and (two) idx + 1.  Rows of odd length put half of the
+// pairs at odd places.  Stored element by element, each store instruction then
+// touched all sectors for half of their bytes: a step of 257^3 D3Q19 fp32 with f,
+// rho and u took 1201 us, with store_run 723 (dense rows, one node per thread: 850).
 template <int Q, int SH>
 __device__ __forceinline__ void observe_pair(const StepArgs &a, const F2 f[Q], unsigned idx,
-                                             bool two, F2 rho, F2 ux, F2 uy, F2 uz) {
-  if (!two || !a.obs_pairs) {
-    float fa[Q], fb[Q];
-    static_for<Q>([&](auto ic) {
-      constexpr int i = decltype(ic)::value;
-      fa[i] = f[i].v.x;
-      fb[i] = f[i].v.y;
-    });
-    observe_node<Q, true, SH>(a, fa, idx, rho.v.x, ux.v.x, uy.v.x, uz.v.x);
-    if (two) observe_node<Q, true, SH>(a, fb, idx + 1, rho.v.y, ux.v.y, uy.v.y, uz.v.y);
+                                             bool two, unsigned lanes, F2 rho, F2 ux, F2 uy,
+                                             F2 uz) {
+  float *of = static_cast<float *>(a.obs_f), *orho = static_cast<float *>(a.obs_rho),
+        *ou = static_cast<float *>(a.obs_u);
+  auto value = [&](int i) {
+    return f[i] * F2(1.f / (float)(1 << SH)) + F2(VSet<Q>::w(i));
+  };
+  if (a.obs_pairs) {   // (every pair whole and at an even place)
+    if (of != nullptr)
+      static_for<Q>([&](auto ic) {
+        constexpr int i = decltype(ic)::value;
+        *reinterpret_cast<float2 *>(of + (long long)i * a.g.n + idx) = value(i).v;
+      });
+    if (orho != nullptr) *reinterpret_cast<float2 *>(orho + idx) = rho.v;
+    if (ou != nullptr) {
+      float2 *d = reinterpret_cast<float2 *>(ou + 3ull * idx);
+      d[0] = make_float2(ux.v.x, uy.v.x);
+      d[1] = make_float2(uz.v.x, ux.v.y);
+      d[2] = make_float2(uy.v.y, uz.v.y);
+    }
     return;
   }
-  if (a.obs_f != nullptr) {
-    float *of = static_cast<float *>(a.obs_f);
+  if (of != nullptr)
     static_for<Q>([&](auto ic) {
       constexpr int i = decltype(ic)::value;
-      const F2 v = f[i] * F2(1.f / (float)(1 << SH)) + F2(VSet<Q>::w(i));
-      *reinterpret_cast<float2 *>(of + (long long)i * a.g.n + idx) = v.v;
+      const F2 v = value(i);
+      store_run(of + (long long)i * a.g.n + idx, v.v.x, v.v.y, two, lanes);
     });
-  }
-  if (a.obs_rho != nullptr)
-    *reinterpret_cast<float2 *>(static_cast<float *>(a.obs_rho) + idx) = rho.v;
-  if (a.obs_u != nullptr) {
-    float2 *ou = reinterpret_cast<float2 *>(static_cast<float *>(a.obs_u) + 3ull * idx);
-    ou[0] = make_float2(ux.v.x, uy.v.x);
-    ou[1] = make_float2(uz.v.x, ux.v.y);
-    ou[2] = make_float2(uy.v.y, uz.v.y);
-  }
+  if (orho != nullptr) store_run(orho + idx, rho.v.x, rho.v.y, two, lanes);
+  if (ou != nullptr) store_run3(ou + 3ull * idx, ux, uy, uz, two, lanes);
 }
 
 // What a launch does with its nodes: advance them (collide and store), write
@@ -204,8 +250,8 @@ __device__ __forceinline__ void finish_node(const StepArgs &a, R f[Q], unsigned 
 // partner: its lane holds padding and reports nothing).
 template <int Q, bool FORCE, int SH, Op OP>
 __device__ __forceinline__ void finish_pair(const StepArgs &a, F2 f[Q], unsigned idx, int x, int y,
-                                            int z, bool row_face, bool two, ChunkForce c0,
-                                            ChunkForce c1, unsigned &bad) {
+                                            int z, bool row_face, bool two, unsigned lanes,
+                                            ChunkForce c0, ChunkForce c1, unsigned &bad) {
   Face2 face;
   face.a = row_face || z == 0 || z == a.g.nz - 1;
   face.b = row_face || z + 1 == a.g.nz - 1;
@@ -234,7 +280,7 @@ __device__ __forceinline__ void finish_pair(const StepArgs &a, F2 f[Q], unsigned
     if (face.a) write_face_rho<Q>(a.g, fr, x, y, z, rho.v.x);
     if (face.b && two) write_face_rho<Q>(a.g, fr, x, y, z + 1, rho.v.y);
   }
-  if constexpr (observes(OP)) observe_pair<Q, SH>(a, f, idx, two, rho, ux, uy, uz);
+  if constexpr (observes(OP)) observe_pair<Q, SH>(a, f, idx, two, lanes, rho, ux, uy, uz);
   if constexpr (advances(OP)) collide_dev<Q, SH>(f, a.g, rho, drho, ux, uy, uz);
 }
 
@@ -571,9 +617,18 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
   static_assert(St::kBits <= 32 && NZ % 2 == 0, "pairs of float32 arithmetic");
   static_assert(ALIGNED || (NZ == 2 && St::kBits == 16), "unaligned pairs are single 16-bit pairs");
   constexpr int kWords = NZ * St::kBits / 32;
-  if (pidx0 >= (unsigned)a.g.np) return;
-  int x, y, z0;
-  a.pdec(pidx0, x, y, z0);
+  int x = 0, y = 0, z0 = 0;
+  unsigned lanes = 0;   // observing: the warp's threads that hold nodes (store_run)
+  if constexpr (observes(OP)) {
+    static_assert(NZ == 2, "a thread observes one pair");
+    const bool inside = pidx0 < (unsigned)a.g.np;
+    if (inside) a.pdec(pidx0, x, y, z0);
+    lanes = __ballot_sync(0xffffffffu, inside && z0 < a.g.nz);
+    if (!inside) return;
+  } else {
+    if (pidx0 >= (unsigned)a.g.np) return;
+    a.pdec(pidx0, x, y, z0);
+  }
   if constexpr (PITCH) {
     if (z0 >= a.g.nz) {                      // row padding only
       if constexpr (advances(OP)) put_padding_vector<Q, S, NZ>(a, pidx0);
@@ -582,9 +637,10 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
   }
   const unsigned idx0 = (unsigned)(x * a.g.ny + y) * (unsigned)a.g.nz + (unsigned)z0;
   const int nv = PITCH && a.g.nz - z0 < NZ ? a.g.nz - z0 : NZ;    // nodes inside the row
-  if (!lbm_in(x < a.g.nx && y < a.g.ny && pidx0 + NZ <= (unsigned)a.g.np &&
-              idx0 + nv <= (unsigned)a.g.n))
-    return;
+  const bool in_bounds = lbm_in(x < a.g.nx && y < a.g.ny && pidx0 + NZ <= (unsigned)a.g.np &&
+                                idx0 + nv <= (unsigned)a.g.n);
+  if constexpr (observes(OP)) lanes = __ballot_sync(lanes, in_bounds);
+  if (!in_bounds) return;
   const bool bottom = z0 == 0, top = z0 + NZ >= a.g.nz;
   const RowFaces rf(a.g, x, y);
   const void *const *src = a.p.src[rf.cls()];
@@ -698,8 +754,8 @@ __device__ __forceinline__ void step_pairs_at(const StepArgs &a, const unsigned 
     if (!PITCH || k0 < nv) {
       const bool s0 = ((idx0 + k0) >> 5) == (idx0 >> 5), s1 = ((idx0 + k1) >> 5) == (idx0 >> 5);
       finish_pair<Q, FORCE, St::kShift, OP>(a, f, idx0 + k0, x, y, z0 + k0, rf.any(),
-                                            !PITCH || k1 < nv, s0 ? cf0 : cf1, s1 ? cf0 : cf1,
-                                            bad);
+                                            !PITCH || k1 < nv, lanes, s0 ? cf0 : cf1,
+                                            s1 ? cf0 : cf1, bad);
     }
     if constexpr (advances(OP)) {
       static_for<Q>([&](auto ic) {
@@ -1232,8 +1288,8 @@ struct StepLauncher {
     else
       force ? go_odd_f<true, 128>(a, s) : go_odd_f<false, 128>(a, s);
   }
-  // Observation launch (Op::kBoth: with the step): two nodes per thread where
-  // the rows allow pairs, whatever the step's own launch shape.
+  // Observation launch (Op::kBoth: with the step): its shape does not depend on
+  // the step's own, but that one node per thread stays one.
   template <Op OP, bool FORCE>
   static void go_observe_f(const StepArgs &a, bool pairs, cudaStream_t s) {
     if constexpr (Storage<S>::kBits != 64) {
@@ -1261,7 +1317,16 @@ struct StepLauncher {
     }
     const uintptr_t at = (uintptr_t)a.obs_f | (uintptr_t)a.obs_rho | (uintptr_t)a.obs_u;
     a.obs_pairs = a.g.n % 2 == 0 && a.g.nz % 2 == 0 && at % 8 == 0;
-    const bool pairs = nodes != 1 && step_shape_ok(2, a.g.pz, bits);
+    // Odd rows (or buffers at odd places) without the step: one node per thread
+    // but for the narrower 16-bit sets.  Measured on B200, us with pairs / one
+    // node per thread, rho and u, then f: D3Q19 fp32 257^3 236 / 223, 419 /
+    // 415, 256 x 256 x 255 230 / 220, 417 / 385; D3Q15 fp32 129^3 37 / 27, 58 /
+    // 46; D3Q27 257 x 129 x 129 fp32 103 / 94, 174 / 161, fp16s 96 / 89, 175 /
+    // 162; fp16s D3Q19 257^3 176 / 220, 361 / 416, D3Q15 129^3 23 / 29, 46 / 47,
+    // D3Q13 bf16s 257^3 142 / 193, 253 / 281.  With the step, pairs win
+    // throughout (D3Q19 fp32 257^3, all fields: 723 / 895).
+    const bool pairs = nodes != 1 && step_shape_ok(2, a.g.pz, bits) &&
+                       (a.obs_pairs || OP == Op::kBoth || (bits == 16 && Q != 27));
     if (force)
       go_observe_f<OP, true>(a, pairs, s);
     else

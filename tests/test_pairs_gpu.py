@@ -188,3 +188,45 @@ def test_coupled_step_refuses_what_it_needs():
         _lib.call("lbm_coupled_step", ctypes.byref(lat.desc), lat.buf[0].data_ptr(),
                   lat.buf[1].data_ptr(), ctypes.byref(make_force()), None, None, ctypes.byref(pt),
                   1.0, 1.0, 0.0, 1.0, 1, None, None, 0, 0, None, None, lat.stream())
+
+
+@pytest.mark.parametrize("storage", ["fp32", "bf16s"])
+@pytest.mark.parametrize("shape", [(6, 5, 33), (5, 9, 3), (4, 6, 35), (7, 4, 129), (5, 6, 32)])
+@pytest.mark.parametrize("pitch", [None, True])
+@pytest.mark.parametrize("step", [False, True])
+def test_observed_fields_at_odd_places(storage, shape, pitch, step):
+    """Pairs of odd rows, and buffers that begin at odd places, against one node
+    per thread; the floats around the buffers keep their values."""
+    from funlbm_b200._lib import LbmObserve
+    from funlbm_b200.lattice import Lattice, tau_float32
+
+    q, n = 15, shape[0] * shape[1] * shape[2]
+    f0 = torch.tensor(smooth_f0(q, shape, 0.05, 9)).cuda().permute(3, 0, 1, 2).reshape(q, -1)
+
+    def fields(nodes, pitch, off):
+        lat = Lattice(q, shape, [W, P, P, P, W, W], tau_float32(0.06), storage=storage, pitch=pitch)
+        lat.init(f0.contiguous())
+        lat.step()
+        lat.set_launch_shape(nodes, 128)
+        out = [torch.full((k * n + 8,), -7.0, device="cuda") for k in (q, 1, 3)]
+        obs = LbmObserve(*(t.data_ptr() + 4 * (off + j) for j, t in enumerate(out)))
+        if step:
+            lat.step(obs=obs)
+        else:
+            lat.step()
+            lat.cur ^= 1
+            from funlbm_b200._lib import call, ctypes, ptr
+
+            call("lbm_flow_step", ctypes.byref(lat.desc), ptr(lat.buf[lat.cur]), None, None, None,
+                 None, ctypes.byref(obs), None, lat.stream())
+        got = []
+        for j, (t, k) in enumerate(zip(out, (q, 1, 3))):
+            lo = off + j
+            got.append(t[lo:lo + k * n].clone())
+            assert bool((t[:lo] == -7).all()) and bool((t[lo + k * n:] == -7).all())
+        return got
+
+    want = fields(1, False, 0)
+    for off in (0, 1, 2):
+        for a, b in zip(want, fields(0, pitch, off)):
+            assert torch.equal(a, b)
