@@ -297,7 +297,9 @@ class FlowD3(Flow):
     # attribute brings up that tensor alone (u and rho come from one launch):
     # writing f costs as many bytes again as reading the populations, p and
     # FOL a pass each, and a program that monitors u and rho asks for none of
-    # them.
+    # them.  f brings u and rho with it: they are 16 bytes a node beside 4 q,
+    # and a second read of the populations if they are asked for later (256^3
+    # D3Q19 fp32: f 380 us, f with u and rho 424, u and rho alone 219).
     _ALL = frozenset(("_f", "_u", "_rou", "_p", "_FOL"))
 
     @property
@@ -319,6 +321,7 @@ class FlowD3(Flow):
             if self._f is None:        # released while stepping in the fused form
                 self._f = torch.empty((self.q, self.n), device=self.device, dtype=lat.real_dtype)
             f = self._f
+            need |= self._stale & {"_u", "_rou"}
         if need & {"_u", "_rou"} or ("_p" in need and "_rou" in self._stale):
             # the kernel writes dense [x][y][z](3) arrays through the raw pointers
             if not self._rou.is_contiguous():

@@ -1,0 +1,38 @@
+"""Fields of the fused form read one after another."""
+import pytest
+import torch
+
+from tests.gpu_util import init_with, lbm_config, require_cuda, run, smooth_f0
+
+pytestmark = pytest.mark.gpu
+W, P = 1200, 11000
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    require_cuda()
+
+
+def _stepped(storage="fp32"):
+    from funlbm_b200.lbm import LBMD3
+
+    lbm = LBMD3(config=lbm_config(19, (12, 10, 14), 0.08, [W, W, P, P, W, W],
+                                  body_force=(1e-5, 0, 0), storage=storage))
+    init_with(lbm, smooth_f0(19, (13, 11, 15), 0.03, 5))
+    run(lbm, 3)
+    return lbm
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s"])
+def test_f_brings_u_and_rho(storage):
+    """f, then u and rho: one read of the populations; the same values as read
+    in another order."""
+    a, b = _stepped(storage), _stepped(storage)
+    calls = []
+    plain = a.flow.lattice.observe
+    a.flow.lattice.observe = lambda *args, **kw: (calls.append(1), plain(*args, **kw))
+    first = [a.flow.f, a.flow.u, a.flow.rou]
+    assert len(calls) == 1
+    rou, u, f = b.flow.rou, b.flow.u, b.flow.f
+    for x, y in zip(first, (f, u, rou)):
+        assert torch.equal(x, y)
