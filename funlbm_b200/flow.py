@@ -161,6 +161,12 @@ class Flow:
                                               self.config.Re, self.config.mu)
 
 
+def _writes(t):
+    """torch's count of the writes to a tensor and its views; None where torch
+    keeps none (tensors made in inference mode)."""
+    return None if t.is_inference() else t._version
+
+
 class FlowD3(Flow):
     """3-D flow on liblbm_b200.so (flow/d3/base.py:57-323)."""
 
@@ -174,6 +180,7 @@ class FlowD3(Flow):
         self._tau_t = None
         self._x = None
         self._fp64 = False
+        self._rou_writes = None     # _writes(rho) when it was last brought up
         self._fol_zero = False      # FOL is known to be zero everywhere
 
     # -- geometry ------------------------------------------------------------
@@ -332,8 +339,15 @@ class FlowD3(Flow):
             need |= {"_u", "_rou"}
         if f is not None or u is not None:
             lat.observe(force, f=f, rho=rho, u=u)
+        if rho is not None:
+            self._rou_writes = _writes(rho)
         if "_p" in need:
-            self._p = self._rou / 3.0
+            rho = self._rou
+            if self._rou_writes is None or _writes(rho) != self._rou_writes:
+                # the caller has written to the rho it read: p is that of the state
+                rho = torch.empty(self.shape + (1,), device=self.device, dtype=lat.real_dtype)
+                lat.observe(force, rho=rho)
+            self._p = rho / 3.0
         if "_FOL" in need:
             self._fol_zero = False
             new_field, new_uniform = fields

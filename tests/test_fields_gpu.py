@@ -36,3 +36,31 @@ def test_f_brings_u_and_rho(storage):
     rou, u, f = b.flow.rou, b.flow.u, b.flow.f
     for x, y in zip(first, (f, u, rou)):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("write", [
+    lambda rou: rou.sub_(1.0),
+    lambda rou: rou[3:, ..., 0].zero_(),
+    lambda rou: rou.view(-1)[::2].fill_(5.0),
+])
+def test_p_of_a_rho_that_was_written_to(write):
+    a, b = _stepped(), _stepped()
+    want = a.flow.p.clone()
+    rou = b.flow.rou
+    kept = rou.clone()
+    write(rou)
+    mine = rou.clone()
+    assert torch.equal(b.flow.p, want)
+    assert torch.equal(want, kept / 3.0)
+    assert torch.equal(b.flow.rou, mine)            # what the caller wrote stays
+    run(b, 1)
+    run(a, 1)
+    assert torch.equal(b.flow.rou, a.flow.rou) and torch.equal(b.flow.p, a.flow.p)
+
+
+def test_p_in_inference_mode():
+    with torch.inference_mode():
+        a, b = _stepped(), _stepped()
+        want = a.flow.p.clone()
+        b.flow.rou.zero_()
+        assert torch.equal(b.flow.p, want)
