@@ -143,8 +143,9 @@ def tune_class_of(q, storage, nz, forced, device="cuda", iters=6, warmup=2):
     _, _, even, by4, by8, _ = key
     pnz = 96 if by8 else 100 if by4 else 98 if even else 97
     n = CLASS_PROXY_NODES
+    # (rows of the class's own length: the default would pad the odd ones)
     proxy = Lattice(int(q), (n, n, pnz), [11000] * 6, tau_float32(0.05), storage=storage,
-                    device=device)
+                    device=device, pitch=False)
     proxy.init(None)
     force, keep = None, None
     if forced:
@@ -185,6 +186,8 @@ def tune_class_of(q, storage, nz, forced, device="cuda", iters=6, warmup=2):
 def tune_class(lat, forced=False):
     """Set ``lat``'s launch shape to its class's tuned choice (tune_class_of)."""
     choice = tune_class_of(lat.q, lat.storage, lat.pz, forced, device=lat.device)
+    if not shape_ok(choice[0], lat.pz, STORAGE_BITS[lat.storage], lat.shape[2]):
+        choice = (1, 256)       # (rows shorter than the class's vectors)
     lat.set_launch_shape(*choice)
     return choice
 
