@@ -252,10 +252,11 @@ class LBMServer:
                 flow = r.config.get("flow") or {}
                 q = int(str(flow.get("param_type") or "D3Q19")[3:])
                 storage = ((flow.get("precision") or {}).get("storage")) or "fp32"
-                pz = default_pz(_shape_of(r.config), storage)
+                shape = _shape_of(r.config)
+                pz = default_pz(shape, storage)
                 forced = bool(r.config.get("particles")) or any(
                     float(v) != 0.0 for v in (flow.get("body_force") or ()))
-                tune_class_of(q, storage, pz, forced, device=self.device)
+                tune_class_of(q, storage, pz, forced, device=self.device, padded=pz != shape[2])
         torch.cuda.synchronize(self.device)
 
     def _tune(self, lbm):

@@ -117,35 +117,37 @@ _CLASS_CACHE = {}
 CLASS_PROXY_NODES = 96          # proxy lattice of a class: about 96^3 nodes
 
 
-def class_key_of(q, storage, pz, forced):
+def class_key_of(q, storage, pz, forced, padded=False):
     """Class of a lattice for the tuner: velocity set, storage, the vector
-    widths its row pitch pz allows, forced or not."""
+    widths its row pitch pz allows, forced or not, rows padded or not (padded
+    rows have other best widths: D3Q19 fp16s 257^3 240 us with pairs, 267 with 4
+    nodes per thread, unpadded 256^3 226 and 229)."""
     return (int(q), storage, pz % 2 == 0 and pz >= 4, pz % 4 == 0 and pz >= 8,
-            pz % 8 == 0 and pz >= 16, bool(forced))
+            pz % 8 == 0 and pz >= 16, bool(forced), bool(padded))
 
 
 def class_key(lat, forced):
-    return class_key_of(lat.q, lat.storage, lat.pz, forced)
+    return class_key_of(lat.q, lat.storage, lat.pz, forced, lat.pz != lat.shape[2])
 
 
-def tune_class_of(q, storage, nz, forced, device="cuda", iters=6, warmup=2):
+def tune_class_of(q, storage, nz, forced, device="cuda", iters=6, warmup=2, padded=False):
     """Launch shape of the class (velocity set, storage, which vector widths
-    rows of nz nodes allow, forced or not), tuned once per class on a ~96^3
-    periodic proxy (forced: force fields in 5 % of the 32-node chunks, as
+    rows of pitch nz allow, forced or not, padded by an element or not), tuned
+    once per class on a ~96^3 periodic proxy (forced: force fields in 5 % of the 32-node chunks, as
     spreading leaves them) and cached.  Meant for servers that see many
     lattice sizes: one short tuning per class instead of one per (ny, nz).
     Returns (nodes, threads)."""
     from .lattice import Lattice, make_force, tau_float32
 
-    key = class_key_of(q, storage, nz, forced)
+    key = class_key_of(q, storage, nz, forced, padded)
     if key in _CLASS_CACHE:
         return _CLASS_CACHE[key]
-    _, _, even, by4, by8, _ = key
-    pnz = 96 if by8 else 100 if by4 else 98 if even else 97
+    even, by4, by8 = key[2:5]
+    ppz = 96 if by8 else 100 if by4 else 98 if even else 97
     n = CLASS_PROXY_NODES
-    # (rows of the class's own length: the default would pad the odd ones)
+    pnz = ppz - 1 if padded else ppz      # (the class's own row layout, not the default one)
     proxy = Lattice(int(q), (n, n, pnz), [11000] * 6, tau_float32(0.05), storage=storage,
-                    device=device, pitch=False)
+                    device=device, pitch=ppz)
     proxy.init(None)
     force, keep = None, None
     if forced:
@@ -176,16 +178,16 @@ def tune_class_of(q, storage, nz, forced, device="cuda", iters=6, warmup=2):
         stop.record()
         stop.synchronize()
         timings[(nodes, threads)] = start.elapsed_time(stop) / iters
-    ppz = proxy.pz
     proxy.release()
     del proxy
-    _CLASS_CACHE[key] = _pick(timings, default_shape(q, storage, ppz, forced))
+    _CLASS_CACHE[key] = _pick(timings, default_shape(q, storage, ppz, forced, padded))
     return _CLASS_CACHE[key]
 
 
 def tune_class(lat, forced=False):
     """Set ``lat``'s launch shape to its class's tuned choice (tune_class_of)."""
-    choice = tune_class_of(lat.q, lat.storage, lat.pz, forced, device=lat.device)
+    choice = tune_class_of(lat.q, lat.storage, lat.pz, forced, device=lat.device,
+                           padded=lat.pz != lat.shape[2])
     if not shape_ok(choice[0], lat.pz, STORAGE_BITS[lat.storage], lat.shape[2]):
         choice = (1, 256)       # (rows shorter than the class's vectors)
     lat.set_launch_shape(*choice)

@@ -84,3 +84,29 @@ def test_tuner_keeps_the_default_within_its_margin():
     assert tune._pick(t, (2, 128)) == (2, 128)          # within 3 %: keep the default
     t[(1, 256)] = 2.9
     assert tune._pick(t, (2, 128)) == (1, 256)          # clearly faster: take it
+
+
+def test_class_keys_tell_padded_rows(monkeypatch):
+    """Padded rows are a class of their own, tuned on padded rows; the proxy has
+    the pitch of its class."""
+    from funlbm_b200 import lattice
+
+    k = tune.class_key_of
+    assert k(19, "fp16s", 100, False, True) != k(19, "fp16s", 100, False)
+    seen = []
+
+    class Stop(Exception):
+        pass
+
+    def proxy(q, shape, *args, pitch=None, **kw):
+        seen.append((shape[2], lattice.pitch_of(pitch, shape, kw["storage"])))
+        raise Stop
+
+    monkeypatch.setattr(lattice, "Lattice", proxy)
+    for pz in (65, 66, 68, 72):
+        for padded in (False, True):
+            with pytest.raises(Stop):
+                tune.tune_class_of(19, "fp16s", pz, False, padded=padded)
+            nz, ppz = seen[-1]
+            assert (ppz != nz) == padded
+            assert k(19, "fp16s", ppz, False, padded) == k(19, "fp16s", pz, False, padded)
