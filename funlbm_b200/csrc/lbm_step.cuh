@@ -1339,7 +1339,9 @@ struct StepLauncher {
     if (a.obs_f != nullptr || a.obs_rho != nullptr || a.obs_u != nullptr)
       return go_observe<Op::kBoth>(a, force, nodes, s);
     if (nodes == LBM_STEP_ROWS) return go_tma(a, force, s);
-    const bool odd_pairs = bits == 16 && a.g.pz % 2 == 1 && a.g.nz >= 3;
+    const bool odd_pairs = bits == 16 && a.g.pz % 2 == 1 && a.g.pz == a.g.nz && a.g.nz >= 3;
+    // (k_step_odd's rows are dense: an odd pitch beyond nz takes one node per thread)
+    if (nodes == 2 && a.g.pz % 2 == 1 && !odd_pairs) nodes = 1;
     if (nodes == 0) {
       // Measured on B200, blocks of 128 threads, fraction of the copy peak for
       // 2 / 4 nodes per thread (256^3 unless said): FP32 D3Q19 1.02 / 1.00

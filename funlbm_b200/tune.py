@@ -36,7 +36,7 @@ def shape_ok(nodes, pz, bits, nz=None):
     if nodes * bits // 32 not in (1, 2, 4):
         return False
     if nodes == 2 and bits == 16 and pz % 2 == 1 and pz >= 3:
-        return True                 # pairs within unpitched rows of odd length
+        return pz == nz             # pairs within unpitched rows of odd length
     return pz % nodes == 0 and pz >= 2 * nodes
 
 

@@ -110,3 +110,7 @@ def test_class_keys_tell_padded_rows(monkeypatch):
             nz, ppz = seen[-1]
             assert (ppz != nz) == padded
             assert k(19, "fp16s", ppz, False, padded) == k(19, "fp16s", pz, False, padded)
+
+
+def test_pairs_of_odd_rows_are_dense():
+    assert tune.shape_ok(2, 35, 16, 35) and not tune.shape_ok(2, 35, 16, 33)

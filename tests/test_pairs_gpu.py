@@ -230,3 +230,14 @@ def test_observed_fields_at_odd_places(storage, shape, pitch, step):
     for off in (0, 1, 2):
         for a, b in zip(want, fields(0, pitch, off)):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("storage", ["fp16s", "bf16s"])
+@pytest.mark.parametrize("nz,pitch", [(33, 35), (32, 33), (4, 7)])
+def test_two_nodes_on_rows_of_odd_pitch(storage, nz, pitch):
+    """Two nodes per thread asked for on padded rows of odd pitch: the same bits
+    as on dense rows."""
+    shape, faces = (6, 5, nz), [W, P, P, W, S, W]
+    dense = _forced_run(19, storage, shape, faces, False, 1, 3)
+    for a, b in zip(dense, _forced_run(19, storage, shape, faces, pitch, 2, 3)):
+        assert np.array_equal(a, b)
