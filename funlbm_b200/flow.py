@@ -182,6 +182,7 @@ class FlowD3(Flow):
         self._fp64 = False
         self._rou_writes = None     # _writes(rho) when it was last brought up
         self._fol_zero = False      # FOL is known to be zero everywhere
+        self._fol_shared = False    # the caller holds FOL: it may write to it at any time
 
     # -- geometry ------------------------------------------------------------
     @property
@@ -227,7 +228,7 @@ class FlowD3(Flow):
         self._rou = torch.ones((X, Y, Z, 1), device=dev)
         self._p = torch.zeros((X, Y, Z, 1), device=dev)
         self._FOL = torch.zeros((X, Y, Z, 3), device=dev)
-        self._fol_zero = True
+        self._fol_zero, self._fol_shared = True, False
         self._scratch = torch.zeros(1, device=dev)
         self._mode = "ref"
         self._obs_valid = True
@@ -349,7 +350,7 @@ class FlowD3(Flow):
                 lat.observe(force, rho=rho)
             self._p = rho / 3.0
         if "_FOL" in need:
-            self._fol_zero = False
+            self._fol_zero = self._fol_shared = False
             new_field, new_uniform = fields
             rdt = lat.real_dtype
             # the uniform force reaches the kernels as float32
@@ -545,14 +546,15 @@ class FlowD3(Flow):
 
     @property
     def FOL(self):
-        self._fol_zero = False      # (the caller may write to it)
-        return self._get("_FOL")
+        fol = self._get("_FOL")
+        self._fol_zero, self._fol_shared = False, True
+        return fol
 
     @FOL.setter
     def FOL(self, value):
-        self._fol_zero = False
         self._set("_FOL", torch.as_tensor(value, dtype=torch.float32, device=self.device)
                   .reshape(self.shape + (3,)).contiguous())
+        self._fol_zero, self._fol_shared = False, True      # (it may be the caller's tensor)
 
     @property
     def feq(self):
@@ -608,7 +610,7 @@ class FlowD3(Flow):
             return
         group.create_dataset("f", data=self.f.cpu().numpy(), compression="gzip",
                              compression_opts=9)
-        group.create_dataset("FOL", data=self.FOL.cpu().numpy(), compression="gzip",
+        group.create_dataset("FOL", data=self._get("_FOL").cpu().numpy(), compression="gzip",
                              compression_opts=9)
         if self._mode == "fused":
             lat = self._lat
@@ -641,6 +643,7 @@ class FlowD3(Flow):
         fol = group.get("FOL")
         if fol is not None:
             self.FOL = torch.tensor(np.asarray(fol[:]), dtype=torch.float32, device=self.device)
+            self._fol_shared = False
         self.update_u_rou()
         if not exact:
             return

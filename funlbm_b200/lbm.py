@@ -289,9 +289,10 @@ class LBMBase:
 
     def _no_force(self):
         """Whether this step has no force anywhere, before and after: no
-        particles, no body force, FOL zero since the last step.  cul_equ2 then
-        adds zeros and the second update_u_rou repeats the first.  (Not when a
-        subclass or an instance replaces one of the methods.)"""
+        particles, no body force, FOL zero since the last step and in no one
+        else's hands.  cul_equ2 then adds zeros and the second update_u_rou
+        repeats the first.  (Not when a subclass or an instance replaces one of
+        the methods.)"""
         return False
 
     def _handle_immersed_boundary(self) -> None:
@@ -633,7 +634,8 @@ class LBMD3(LBMBase):
         fl = self.flow
         fl._to_ref()
         fl._FOL.zero_()
-        fl._fol_zero = not self.particle_swarm.particles and self.body_force == (0.0, 0.0, 0.0)
+        fl._fol_zero = (not fl._fol_shared and not self.particle_swarm.particles
+                        and self.body_force == (0.0, 0.0, 0.0))
         parts = self.particle_swarm.particles
         if parts:
             if not hasattr(self, "_ref_chunks"):

@@ -64,3 +64,50 @@ def test_p_in_inference_mode():
         want = a.flow.p.clone()
         b.flow.rou.zero_()
         assert torch.equal(b.flow.p, want)
+
+
+@pytest.mark.parametrize("when", ["before", "between"])
+def test_force_field_written_through_a_kept_reference(when):
+    """Reference call sequence: FOL taken before or between steps and written to
+    in place is cleared within the next step, as when no pass is skipped."""
+    from funlbm_b200.lbm import LBMD3
+
+    def stepped(skip):
+        lbm = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+        init_with(lbm, smooth_f0(19, (10, 7, 8), 0.02, 2))
+        if not skip:
+            lbm._no_force = lambda: False
+        if when == "between":
+            run(lbm, 2)
+        fol = lbm.flow.FOL
+        run(lbm, 3)
+        states = []
+        for _ in range(3):
+            fol.fill_(1e-4)
+            run(lbm, 1)
+            states += [lbm.flow.f.clone(), lbm.flow.u.clone(), lbm.flow.rou.clone(), fol.clone()]
+        return states
+
+    for a, b in zip(stepped(True), stepped(False)):
+        assert torch.equal(a, b)
+
+
+def test_forcing_is_skipped_until_the_force_field_is_handed_out(tmp_path):
+    from funlbm_b200.lbm import LBMD3, _NpzGroup
+
+    lbm = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+    lbm.init()
+    run(lbm, 2)
+    assert lbm._no_force()
+    store = _NpzGroup()
+    lbm.dump_checkpoint(store)                      # (reads FOL, hands nothing out)
+    run(lbm, 1)
+    assert lbm._no_force()
+    other = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+    other.init()
+    other.load_checkpoint(group=store)
+    run(other, 1)
+    assert other._no_force()
+    lbm.flow.FOL
+    run(lbm, 2)
+    assert not lbm._no_force()
