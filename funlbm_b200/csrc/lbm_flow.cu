@@ -146,24 +146,32 @@ __device__ __forceinline__ void atomic_max_nonneg(float *addr, float v) {
 
 // Moments of one node to the fields, and the block's greatest density to rmax.
 // Called by every thread of the block (inside: the node exists).
+// settle: these are the step's last moments, since there is no force.  Adding a
+// force of zero changes nothing but at a node whose velocity is not finite:
+// every population of such a node becomes NaN, and its moments with them.
+// Returns whether that holds here (the caller writes the populations).
 template <int Q>
-__device__ __forceinline__ void write_moments(const Geom &g, bool inside, const float f[Q],
+__device__ __forceinline__ bool write_moments(const Geom &g, bool inside, const float f[Q],
                                               const float *fol, unsigned idx, int x, int y, int z,
-                                              float *rho, float *u, float *p, float *rmax) {
+                                              float *rho, float *u, float *p, float *rmax,
+                                              bool settle = false) {
   __shared__ float s_max[kThreads / 32];
   float r = 0.f;
+  bool lost = false;
   if (inside) {
     const float fx = fol ? fol[3ull * idx] : 0.f, fy = fol ? fol[3ull * idx + 1] : 0.f,
                 fz = fol ? fol[3ull * idx + 2] : 0.f;
     float ux, uy, uz;
     moments<Q>(f, fx, fy, fz, on_any_face(g, x, y, z), r, ux, uy, uz);
+    lost = settle && !(isfinite(ux) && isfinite(uy) && isfinite(uz));
+    if (lost) r = ux = uy = uz = NAN;
     rho[idx] = r;
     if (p != nullptr) p[idx] = r / 3.0f;
     u[3ull * idx] = ux;
     u[3ull * idx + 1] = uy;
     u[3ull * idx + 2] = uz;
   }
-  if (rmax == nullptr) return;  // uniform per launch
+  if (rmax == nullptr) return lost;  // uniform per launch
   for (int o = 16; o > 0; o >>= 1) r = fmaxf(r, __shfl_xor_sync(0xffffffffu, r, o));
   if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = r;
   __syncthreads();
@@ -172,6 +180,7 @@ __device__ __forceinline__ void write_moments(const Geom &g, bool inside, const 
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (threadIdx.x == 0) atomic_max_nonneg(rmax, m);
   }
+  return lost;
 }
 
 template <int Q>
@@ -192,7 +201,8 @@ __global__ void __launch_bounds__(kThreads)
 }
 
 // f_stream and the update_u_rou after it in one pass: the streamed
-// populations are still in registers when their moments are taken.
+// populations are still in registers when their moments are taken.  Without
+// fol the step has no force and ends here (write_moments: settle).
 template <int Q>
 __global__ void __launch_bounds__(kThreads)
     k_stream_moments(const __grid_constant__ Geom g, const NodeDecomp dec,
@@ -211,26 +221,45 @@ __global__ void __launch_bounds__(kThreads)
       static_cast<float *>(pl.dst[i])[idx] = f[i];
     });
   }
-  write_moments<Q>(g, inside, f, fol, idx, x, y, z, rho, u, p, rmax);
+  if (write_moments<Q>(g, inside, f, fol, idx, x, y, z, rho, u, p, rmax, fol == nullptr)) {
+    static_for<Q>([&](auto ic) {
+      constexpr int i = decltype(ic)::value;
+      static_cast<float *>(pl.dst[i])[idx] = NAN;
+    });
+  }
 }
 
 // update_u_rou_boundary's NON_EQUILIBRIUM part (flow/d3/base.py:135-148): the
 // inlet takes the duct profile scaled by Re mu / max(rho) / min(Y, Z) and the
 // density of plane 1; the outlet copies plane X-2.  One thread per (y, z).
-__global__ void k_neq_moments(const Geom g, float *rho, float *u, const float *rmax) {
+// With f (q populations; p may be NULL) as in write_moments' settle: a node whose
+// velocity comes out not finite loses its populations.
+__global__ void k_neq_moments(const Geom g, float *rho, float *u, const float *rmax, float *f,
+                              int q, float *p) {
   chain_enter();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.nyz) return;
   const long long plane = g.nyz;
+  auto lose = [&](long long idx) {
+    for (int i = 0; i < q; ++i) f[(long long)i * g.n + idx] = NAN;
+    if (p != nullptr) p[idx] = NAN;
+  };
   if (g.face[0] == LBM_BC_NON_EQUILIBRIUM) {
     const float uw = (1.0f / *rmax) * g.re_mu / (float)(g.ny < g.nz ? g.ny : g.nz);
-    u[3 * t] = (float)((double)uw * g.neq_profile[t]);
+    const float ux = (float)((double)uw * g.neq_profile[t]);
+    u[3 * t] = ux;
     rho[t] = rho[plane + t];
+    if (f != nullptr && !isfinite(ux)) lose(t);
   }
   if (g.face[1] == LBM_BC_NON_EQUILIBRIUM) {
     const long long last = (long long)(g.nx - 1) * plane + t, prev = last - plane;
     rho[last] = rho[prev];
-    for (int k = 0; k < 3; ++k) u[3 * last + k] = u[3 * prev + k];
+    bool finite = true;
+    for (int k = 0; k < 3; ++k) {
+      u[3 * last + k] = u[3 * prev + k];
+      finite = finite && isfinite(u[3 * prev + k]);
+    }
+    if (f != nullptr && !finite) lose(last);
   }
 }
 
@@ -584,7 +613,8 @@ int lbm_moments(const lbm_lattice *lat, const float *f, const float *fol, float 
   }
   rc = dispatch_q<RunMoments>(lat->q, g, f, fol, rho, u, p, neq_in ? scratch : nullptr, s);
   if (rc || !neq) return rc;
-  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch);
+  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch, nullptr, 0,
+                 nullptr);
   LBM_LAUNCH_CHECK("lbm_moments");
   return LBM_OK;
 }
@@ -613,7 +643,8 @@ int lbm_compute_flow(const lbm_lattice *lat, float *f, float *f_out, const float
                                     static_cast<const float *>(feq), fol, rho, u, p,
                                     neq_in ? scratch : nullptr, s);
   if (rc || !any_face(lat, LBM_BC_NON_EQUILIBRIUM)) return rc;
-  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch);
+  launch_chained(k_neq_moments, blocks_for(g.nyz, 128), 128, 0, s, g, rho, u, scratch,
+                 fol == nullptr ? f_out : nullptr, lat->q, p);
   LBM_LAUNCH_CHECK("lbm_compute_flow");
   return LBM_OK;
 }

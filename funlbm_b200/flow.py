@@ -470,16 +470,18 @@ class FlowD3(Flow):
             getattr(cls, k) is getattr(FlowD3, k) and k not in self.__dict__
             for k in self._STEP_METHODS)
 
-    def compute_flow(self, step=0):
-        """cul_equ, f_stream and update_u_rou in one call (lbm/base.py:159-163)."""
+    def compute_flow(self, step=0, force=True):
+        """cul_equ, f_stream and update_u_rou in one call (lbm/base.py:159-163);
+        force=False (FOL zero and no other force in this step): the state is that
+        after cul_equ2 and the second update_u_rou, too."""
         self._to_ref()
         if self._feq is None:
             self._feq = torch.empty_like(self._f)
         if self._f2 is None:
             self._f2 = torch.empty_like(self._f)
         call("lbm_compute_flow", ctypes_ref(self._lat.desc_fp32), ptr(self._f), ptr(self._f2),
-             ptr(self._FOL), ptr(self._rou), ptr(self._u), ptr(self._p), ptr(self._feq),
-             ptr(self._scratch), self._lat.stream())
+             ptr(self._FOL) if force else None, ptr(self._rou), ptr(self._u), ptr(self._p),
+             ptr(self._feq), ptr(self._scratch), self._lat.stream())
         self._f, self._f2 = self._f2, self._f
 
     def update_u_rou_boundary(self, *args, **kwargs):

@@ -281,7 +281,7 @@ class LBMBase:
     # -- reference call sequence -----------------------------------------------
     def _compute_flow(self) -> None:
         if self.flow._plain_methods():
-            self.flow.compute_flow(step=self.step)
+            self.flow.compute_flow(step=self.step, force=not self._no_force())
             return
         self.flow.cul_equ(step=self.step)
         self.flow.f_stream()
@@ -291,7 +291,7 @@ class LBMBase:
         """Whether this step has no force anywhere, before and after: no
         particles, no body force, FOL zero since the last step and in no one
         else's hands.  cul_equ2 then adds zeros and the second update_u_rou
-        repeats the first.  (Not when a subclass or an instance replaces one of
+        repeats the first; compute_flow(force=False) ends the step.  (Not when a subclass or an instance replaces one of
         the methods.)"""
         return False
 

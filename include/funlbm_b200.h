@@ -211,8 +211,9 @@ int lbm_moments(const lbm_lattice *lat, const float *f, const float *fol, float 
 /* cul_equ, f_stream and update_u_rou in one call (LBMBase._compute_flow,
  * lbm/base.py:159-163): collides f in place and writes feq, streams f into
  * f_out and takes the moments there with FOL = fol -- the results of
- * lbm_collide, lbm_stream and lbm_moments one after the other.  p may be NULL;
- * scratch: one float. */
+ * lbm_collide, lbm_stream and lbm_moments one after the other.  fol = NULL: the
+ * step has no force, and the results are those after lbm_add_force and the
+ * second lbm_moments with FOL = 0.  p may be NULL; scratch: one float. */
 int lbm_compute_flow(const lbm_lattice *lat, float *f, float *f_out, const float *fol, float *rho,
                      float *u, float *p, float *feq, float *scratch, void *stream);
 /* FlowD3.cul_equ2 (flow/d3/base.py:103-114): f += forcing(u, FOL) in place. */

@@ -111,3 +111,37 @@ def test_forcing_is_skipped_until_the_force_field_is_handed_out(tmp_path):
     lbm.flow.FOL
     run(lbm, 2)
     assert not lbm._no_force()
+
+
+@pytest.mark.parametrize("q", [13, 19, 27])
+@pytest.mark.parametrize("faces", [[1400, 1400, W, W, W, W], [1400, W, P, P, W, W],
+                                   [P, P, W, W, P, P], [W, W, W, W, W, 1201]])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf"), "empty"])
+def test_steps_without_force_keep_what_is_not_finite(q, faces, bad):
+    """Populations that are not finite, and nodes of density zero, spread in the
+    steps that skip the forcing as they do through it."""
+    from funlbm_b200.lbm import LBMD3
+
+    shape = (10, 7, 8)
+
+    def stepped(skip):
+        lbm = LBMD3(config=lbm_config(q, (9, 6, 7), 0.1, faces, uw=[(0.0, 0.01, 0.0)] * 6,
+                                      fused=False))
+        f0 = torch.tensor(smooth_f0(q, shape, 0.02, 2))
+        for k, at in enumerate([(4, 3, 4), (8, 3, 3), (1, 2, 2), (0, 3, 5)]):
+            if bad == "empty":
+                f0[at] = 0.0
+            else:
+                f0[at][3 + k] = bad
+        init_with(lbm, f0.numpy())
+        if not skip:
+            lbm._no_force = lambda: False
+        states = []
+        for _ in range(3):
+            run(lbm, 1)
+            states += [getattr(lbm.flow, k).clone() for k in ("f", "u", "rou", "p")]
+        return states
+
+    for k, (a, b) in enumerate(zip(stepped(True), stepped(False))):
+        assert torch.equal(torch.isnan(a), torch.isnan(b)), k
+        assert torch.equal(torch.nan_to_num(a, nan=0.0), torch.nan_to_num(b, nan=0.0)), k
