@@ -459,16 +459,10 @@ class FlowD3(Flow):
         call("lbm_moments", ctypes_ref(self._lat.desc_fp32), ptr(self._f), ptr(self._FOL),
              ptr(self._rou), ptr(self._u), ptr(self._p), ptr(self._scratch), self._lat.stream())
 
-    # the methods that one step of the reference's call sequence runs
-    _STEP_METHODS = ("cul_equ", "f_stream", "update_u_rou", "cul_equ2")
-
     def _plain_methods(self):
-        """Whether the step methods are this class's own (a subclass or an
-        instance may replace them, and is then called one by one)."""
-        cls = type(self)
-        return not self._fp64 and all(
-            getattr(cls, k) is getattr(FlowD3, k) and k not in self.__dict__
-            for k in self._STEP_METHODS)
+        """Whether the step methods are this class's own (a replaced one is
+        called, and then all of them one by one)."""
+        return not self._fp64 and unreplaced(self, _STEP_METHODS)
 
     def compute_flow(self, step=0, force=True):
         """cul_equ, f_stream and update_u_rou in one call (lbm/base.py:159-163);
@@ -663,6 +657,18 @@ class FlowD3(Flow):
         self._mode = "fused"
         self._obs_valid = True
         self._loaded_fused = True       # the next step enters this state's FOL
+
+
+def unreplaced(obj, own):
+    """Whether `obj` runs the functions `own` (by name), none of them replaced in
+    a subclass, on the instance or on the class itself."""
+    cls = type(obj)
+    return own.keys().isdisjoint(obj.__dict__) and all(
+        getattr(cls, name) is fn for name, fn in own.items())
+
+
+# the methods that one step of the reference's call sequence runs, as defined here
+_STEP_METHODS = {k: FlowD3.__dict__[k] for k in ("cul_equ", "f_stream", "update_u_rou", "cul_equ2")}
 
 
 def face_planes(rho3):

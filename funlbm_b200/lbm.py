@@ -41,7 +41,7 @@ import torch
 from . import _lib
 from ._lib import addr, call, ptr
 from .config import BaseConfig, FileConfig, deep_get
-from .flow import FlowConfig, FlowD3, create_flow
+from .flow import FlowConfig, FlowD3, create_flow, unreplaced
 from .lattice import ctypes_ref, make_force
 from .particle import ParticleConfig, ParticleSwarm, create_particle_swarm
 from .steplog import StepLogWriter, StepStore, particle_log_tensor
@@ -602,14 +602,10 @@ class LBMD3(LBMBase):
             self._fi ^= 1
         self._g_old = plan["g_new"]
 
-    _COUPLING = ("flow_to_lagrange", "particle_to_wall", "lagrange_to_flow")
-
     def _no_force(self):
-        cls = type(self)
         return (not self.particle_swarm.particles and self.body_force == (0.0, 0.0, 0.0)
                 and self.flow._fol_zero and self.flow._plain_methods()
-                and all(getattr(cls, k) is getattr(LBMD3, k) and k not in self.__dict__
-                        for k in self._COUPLING))
+                and unreplaced(self, _COUPLING))
 
     # -- reference-mode IBM methods (lbm/lbm3d.py:66-167) -------------------------
     def flow_to_lagrange(self, *args, **kwargs):
@@ -677,6 +673,10 @@ class LBMD3(LBMBase):
         if self._status_ibm is None:
             self._status_ibm = torch.zeros(1, dtype=torch.int32, device=self.device)
 
+
+# the coupling methods of the reference's call sequence, as defined here
+_COUPLING = {k: LBMD3.__dict__[k] for k in ("flow_to_lagrange", "particle_to_wall",
+                                            "lagrange_to_flow")}
 
 _EMPTY = None
 

@@ -145,3 +145,37 @@ def test_steps_without_force_keep_what_is_not_finite(q, faces, bad):
     for k, (a, b) in enumerate(zip(stepped(True), stepped(False))):
         assert torch.equal(torch.isnan(a), torch.isnan(b)), k
         assert torch.equal(torch.nan_to_num(a, nan=0.0), torch.nan_to_num(b, nan=0.0)), k
+
+
+def _counted(calls, name, method):
+    def call(self, *args, **kw):
+        calls.append(name)
+        return method(self, *args, **kw)
+    return call
+
+
+@pytest.mark.parametrize("name", ["cul_equ", "f_stream", "update_u_rou", "cul_equ2"])
+def test_flow_methods_replaced_on_the_class_are_called(monkeypatch, name):
+    from funlbm_b200.flow import FlowD3
+    from funlbm_b200.lbm import LBMD3
+
+    lbm = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+    lbm.init()
+    run(lbm, 1)
+    calls = []
+    monkeypatch.setattr(FlowD3, name, _counted(calls, name, getattr(FlowD3, name)))
+    run(lbm, 3)
+    assert len(calls) == (6 if name == "update_u_rou" else 3)
+
+
+@pytest.mark.parametrize("name", ["flow_to_lagrange", "particle_to_wall", "lagrange_to_flow"])
+def test_coupling_methods_replaced_on_the_class_are_called(monkeypatch, name):
+    from funlbm_b200.lbm import LBMD3
+
+    lbm = LBMD3(config=lbm_config(19, (9, 6, 7), 0.1, [1400, 1400, W, W, W, W]))
+    lbm.init()
+    run(lbm, 1)
+    calls = []
+    monkeypatch.setattr(LBMD3, name, _counted(calls, name, getattr(LBMD3, name)))
+    run(lbm, 3)
+    assert len(calls) == 3
