@@ -42,7 +42,7 @@ from . import _lib
 from ._lib import addr, call, ptr
 from .config import BaseConfig, FileConfig, deep_get
 from .flow import FlowConfig, FlowD3, create_flow, unreplaced
-from .lattice import ctypes_ref, make_force
+from .lattice import Lattice, ctypes_ref, make_force
 from .particle import ParticleConfig, ParticleSwarm, create_particle_swarm
 from .steplog import StepLogWriter, StepStore, particle_log_tensor
 
@@ -503,7 +503,8 @@ class LBMD3(LBMBase):
         """A step with particles and claimed spreading in one library call
         (lbm_coupled_step: fused_prepare's launches and the step kernel), once
         the state is in the fused form and the IBM buffers exist.  Returns
-        False when the step has to take the general way.  The host time of a
+        False when the step has to take the general way, also where one of that
+        way's methods has been replaced.  The host time of a
         particle step was 4 calls, 5 stream look-ups and 2 force structs."""
         fl, sw = self.flow, self.particle_swarm
         if (not sw.particles or self._fol is None or fl._mode != "fused"
@@ -511,6 +512,9 @@ class LBMD3(LBMBase):
                 or self.config.ibm_spread == "tiles"):
             return False
         lat, cfg = fl._lat, self.config
+        if not (unreplaced(self, _FUSED) and unreplaced(fl, _FUSED_FLOW)
+                and unreplaced(lat, _FUSED_LATTICE)):
+            return False
         g_old, g_new = self._g_old, self.body_force
         new, old = self._fi, self._fi ^ 1
         keep = (self._fol[old], self._fol[new], self._chunks[old], self._chunks[new])
@@ -677,6 +681,11 @@ class LBMD3(LBMBase):
 # the coupling methods of the reference's call sequence, as defined here
 _COUPLING = {k: LBMD3.__dict__[k] for k in ("flow_to_lagrange", "particle_to_wall",
                                             "lagrange_to_flow")}
+
+# the methods a fused step goes through, as defined in the package
+_FUSED = {k: LBMD3.__dict__[k] for k in ("fused_prepare", "fused_finish")}
+_FUSED_FLOW = {k: FlowD3.__dict__[k] for k in ("enter_fused", "fused_step")}
+_FUSED_LATTICE = {"step": Lattice.__dict__["step"]}
 
 _EMPTY = None
 

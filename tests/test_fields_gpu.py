@@ -179,3 +179,38 @@ def test_coupling_methods_replaced_on_the_class_are_called(monkeypatch, name):
     monkeypatch.setattr(LBMD3, name, _counted(calls, name, getattr(LBMD3, name)))
     run(lbm, 3)
     assert len(calls) == 3
+
+
+@pytest.mark.parametrize("how", ["class", "subclass", "instance"])
+@pytest.mark.parametrize("owner,name", [("lbm", "fused_prepare"), ("lbm", "fused_finish"),
+                                        ("flow", "enter_fused"), ("flow", "fused_step"),
+                                        ("lattice", "step")])
+def test_step_methods_replaced_in_particle_runs_are_called(monkeypatch, owner, name, how):
+    """A particle step goes through the methods of the fused step when one of
+    them is replaced, with the same results."""
+    from funlbm_b200.lbm import LBMD3
+
+    def make():
+        lbm = LBMD3(config=lbm_config(19, (24, 18, 20), 0.08, [W, W, P, P, W, W], gl=1e-3,
+                                      particles=[{"type": "sphere", "r": 3, "rou": 1.4,
+                                                  "coord": {"center": [12, 9, 10]}}]))
+        lbm.init()
+        run(lbm, 2)
+        return lbm
+
+    a, b = make(), make()
+    run(a, 3)
+    obj = {"lbm": b, "flow": b.flow, "lattice": b.flow.lattice}[owner]
+    calls = []
+    cls = type(obj)
+    counted = _counted(calls, name, getattr(cls, name))
+    if how == "class":
+        monkeypatch.setattr(cls, name, counted)
+    elif how == "subclass":
+        obj.__class__ = type("Own", (cls,), {name: counted})
+    else:
+        monkeypatch.setattr(obj, name, lambda *args, **kw: counted(obj, *args, **kw))
+    run(b, 3)
+    assert len(calls) == 3
+    assert torch.equal(a.flow.u, b.flow.u)
+    assert torch.equal(a.particle_swarm.lx, b.particle_swarm.lx)
