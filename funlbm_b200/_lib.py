@@ -198,11 +198,11 @@ def addr(t):
 
 
 def stream_of(torch_mod, device=None):
-    """Handle of the current CUDA stream of `device` (a torch.device; None or
-    one without an index: the current device)."""
-    index = getattr(device, "index", None)
+    """Handle of the current CUDA stream of `device` (None or a torch.device
+    without an index: the current device)."""
+    if device is not None and not isinstance(device, torch_mod.device):
+        return ctypes.c_void_p(torch_mod.cuda.current_stream(device).cuda_stream)
+    index = None if device is None else device.index
     if index is None:
-        if device is not None and not isinstance(device, torch_mod.device):
-            return ctypes.c_void_p(torch_mod.cuda.current_stream(device).cuda_stream)
         index = torch_mod.cuda.current_device()
     return ctypes.c_void_p(torch_mod._C._cuda_getCurrentRawStream(index))
