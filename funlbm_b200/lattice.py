@@ -60,10 +60,11 @@ def row_pitch(nz, storage):
 
 def pitch_of(pitch, shape, storage):
     """Row pitch in elements for a ``pitch`` argument: None = the default,
-    False = dense rows, True = the vector width, a number = that pitch."""
+    False = dense rows, True = the vector width, a number = that pitch (1 and
+    numpy's truth values count as True: no row has one element)."""
     if pitch is None:
         return default_pz(shape, storage)
-    if pitch is True:
+    if pitch == 1:
         return row_pitch(shape[2], storage)
     return int(pitch) if pitch else int(shape[2])
 

@@ -35,3 +35,14 @@ class _Torch:
 ])
 def test_stream_of_any_device_argument(device, stream):
     assert _lib.stream_of(_Torch, device).value == stream
+
+
+@pytest.mark.parametrize("pitch,pz", [
+    (None, 34), (True, 40), (np.bool_(True), 40), (1, 40), (False, 33), (np.bool_(False), 33),
+    (0, 33), (35, 35), (np.int64(48), 48),
+])
+def test_pitch_arguments(pitch, pz):
+    from funlbm_b200.lattice import pitch_of
+
+    got = pitch_of(pitch, (6, 5, 33), "fp16s")
+    assert got == pz and type(got) is int
