@@ -424,22 +424,30 @@ struct StatAcc {
   double sm[3];
 };
 
-// sum of v[0..N) as a rounded sum and its error, added to `acc`.  The
-// conversion of every value to double was what bounded the kernel (a quarter
-// of the float64 rate): here each addition's error is recovered in float32
-// (|s| >= |v|: the rest population comes first and is the largest) and two
-// values are converted per node.
+// sum of v[0..N), added to `acc`.  The conversion of every value to double was
+// what bounded the kernel (a quarter of the float64 rate): here the even and
+// the odd values are summed in packed float32 with the error of each addition
+// (Knuth's two-sum, exact whichever term is the larger), and four values are
+// converted per node.
 template <int N>
 __device__ __forceinline__ void add_all(const float v[N], double &acc) {
-  float s = v[0], e = 0.f;
+  F2 s(v[0], v[1]), e(0.f);
 #pragma unroll
-  for (int i = 1; i < N; ++i) {
-    const float t = s + v[i];
-    e += v[i] - (t - s);
+  for (int i = 2; i < N; i += 2) {
+    const F2 x(v[i], i + 1 < N ? v[i + 1 < N ? i + 1 : i] : 0.f);
+    const F2 t = s + x;
+    const F2 w = t - s;                // the part of x that t holds
+    e += (s - (t - w)) + (x - w);
     s = t;
   }
-  acc += (double)s;
-  if (fabsf(s) < 3.0e38f) acc += (double)e;   // (an infinite sum has no error term)
+  if (fabsf(s.v.x) + fabsf(s.v.y) < 3.0e38f) {
+    acc += (double)s.v.x;
+    acc += (double)s.v.y;
+    acc += (double)(e.v.x + e.v.y);
+  } else {                             // (sums without an error term)
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc += (double)v[i];
+  }
 }
 template <int N>
 __device__ __forceinline__ void add_all(const double v[N], double &acc) {
@@ -447,8 +455,8 @@ __device__ __forceinline__ void add_all(const double v[N], double &acc) {
   for (int i = 0; i < N; ++i) acc += v[i];
 }
 
-// Resident blocks per SM of k_stats, also its grid (5 blocks of D3Q19 spill
-// and take 66.5 us where 4 take 64.5).
+// Resident blocks per SM of k_stats, also its grid (5 blocks of D3Q19 spilled
+// and took 3 % longer than 4).
 template <int Q, int S>
 constexpr int stats_blocks() {
   return Storage<S>::kBits == 64 ? 2 : Q == 27 ? 3 : 4;
@@ -457,7 +465,8 @@ constexpr int stats_blocks() {
 // Bound by the read of the populations (D3Q19 fp32 193 x 161 x 129: 305 MB, 47
 // us at the copy peak); float32 extremes and the sums above took the registers
 // from 80 to 64 (4 resident blocks instead of 3) and the three launches of
-// lbm_flow_stats from 98 to 65 us.
+// lbm_flow_stats from 99 to 70 us (65 with sums that are exact only while the rest
+// population is the largest).
 template <int Q, int S, bool FORCE>
 __global__ void __launch_bounds__(kStatsThreads, (stats_blocks<Q, S>()))
     k_stats(const __grid_constant__ StepArgs a, unsigned long long *out) {

@@ -186,3 +186,28 @@ def test_save_bak_writes_vtk_and_tecplot(tmp_path):
     row = lines[3 + 1].split()                 # node x=1, y=0, z=0
     assert [int(v) for v in row[:3]] == [1, 0, 0]
     assert np.allclose([float(v) for v in row[3:]], u[1, 0, 0], rtol=1e-6, atol=1e-12)
+
+
+@pytest.mark.parametrize("q,storage", [(13, "bf16s"), (15, "fp16s"), (19, "fp32"), (27, "fp32")])
+def test_step_stats_of_a_field_far_from_equilibrium(q, storage):
+    """The mean of f keeps float64's accuracy where the rest population is not
+    the largest.  Bound: each of a node's q - 1 additions leaves an error of at
+    most 2^-24 of the sum, recovered exactly and summed in float32, so
+    q^2 2^-48 of the populations' mean magnitude."""
+    import torch
+
+    from funlbm_b200.lattice import Lattice
+
+    shape = (33, 29, 31)
+    lat = Lattice(q, shape, [11000] * 6, 0.65, storage=storage)
+    f0 = torch.rand(q, lat.n, generator=torch.Generator().manual_seed(1)) ** 6
+    f0[0] *= 1e-3
+    f0[1:4] *= 3
+    lat.init(f0.cuda())
+    lat.step()
+    f = torch.empty(q, lat.n, device="cuda")
+    lat.observe(None, f=f)
+    f = f.double()
+    mean = float(lat.stats(None)[1])
+    want, scale = (float(t.sum()) / (q * lat.n) for t in (f, f.abs()))
+    assert abs(mean - want) <= q * q * 2.0 ** -48 * scale
