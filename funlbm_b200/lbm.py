@@ -408,6 +408,7 @@ class LBMD3(LBMBase):
     def __init__(self, *args, **kwargs):
         super().__init__(*args, **kwargs)
         self._status_ibm = None
+        self._boxes, self._boxes_due = None, False
 
     def _init(self):
         """lbm/lbm3d.py:23-30"""
@@ -442,7 +443,7 @@ class LBMD3(LBMBase):
         else:
             # claim array of the global-claim spreading, -1 between calls
             self._owner = torch.full((n,), -1, dtype=torch.int32, device=dev)
-        self._boxes = self._make_boxes()
+        self._boxes, self._boxes_due = None, True
         self._fi = 0          # index of the buffer the next spread writes
         self._status_ibm = torch.zeros(1, dtype=torch.int32, device=dev)
         # FOL of the state being entered (zero after init): the next step's
@@ -459,6 +460,9 @@ class LBMD3(LBMBase):
         plan = self.fused_prepare()
         self.flow.fused_step(plan["force"], plan["new_field"], plan["g_new"], keep=plan["keep"])
         self.fused_finish(plan)
+        if self._boxes_due:      # (the entering step, never captured; not where steps are packed)
+            self._boxes_due = False
+            self._boxes = self._make_boxes()
 
     # Markers from which the moments around the particles are taken once per
     # node (lbm_coupled_step's scratch): below, the extra launch costs what it
@@ -481,11 +485,13 @@ class LBMD3(LBMBase):
         return cells if count * cells <= 64 * lagrange.shape[0] else 0
 
     def _make_boxes(self):
-        """lbm_coupled_step's scratch, allocated with the IBM buffers: (buffer,
-        cells per particle, particles), or None when there are few markers or
-        the boxes would be too large."""
+        """lbm_coupled_step's scratch: (buffer, cells per particle, particles), or
+        None when there are few markers, the boxes would be too large or the
+        steps take another form."""
         sw = self.particle_swarm
         count = len(sw.particles)
+        if self.config.ibm_mode != "reference" or self.config.ibm_spread == "tiles":
+            return None
         if not count or sw.n_markers < max(1, self._BOX_MARKERS):
             return None
         cells = self._box_cells(sw.lagrange, count)

@@ -214,3 +214,30 @@ def test_step_methods_replaced_in_particle_runs_are_called(monkeypatch, owner, n
     assert len(calls) == 3
     assert torch.equal(a.flow.u, b.flow.u)
     assert torch.equal(a.particle_swarm.lx, b.particle_swarm.lx)
+
+
+@pytest.mark.parametrize("how,made", [("run_step", True), ("run_steps", True), ("packed", False),
+                                      ("accumulate", False)])
+def test_boxes_are_allocated_for_the_steps_that_use_them(how, made):
+    """The scratch of the node moments belongs to the combined particle step;
+    steps packed with other lattices and the accumulating mode do without."""
+    from funlbm_b200.lbm import LBMD3
+
+    lbm = LBMD3(config=lbm_config(19, (24, 18, 20), 0.08, [W, W, P, P, W, W], gl=1e-3,
+                                  ibm_mode="accumulate" if how == "accumulate" else "reference",
+                                  particles=[{"type": "sphere", "r": 4, "rou": 1.4,
+                                              "coord": {"center": [12, 9, 10]}}]))
+    lbm._BOX_MARKERS = 1
+    lbm.init()
+    if how == "packed":
+        for _ in range(3):
+            plan = lbm.fused_prepare()
+            lbm.flow.fused_step(plan["force"], plan["new_field"], plan["g_new"], keep=plan["keep"])
+            lbm.fused_finish(plan)
+            lbm.step += 1
+    elif how == "run_steps":
+        lbm.run_steps(40)
+    else:
+        run(lbm, 3)
+    assert (lbm._boxes is not None) == made
+    assert float(lbm.flow.u.abs().max()) > 0 and lbm.check_status() == 0
