@@ -73,10 +73,28 @@ def _q_storage(cfg):
     return q, storage
 
 
+def _box_bytes(cfg, real):
+    """Most that the boxes of node moments around the particles can take
+    (LBMD3._make_boxes, sized from the bodies' largest half axis instead of
+    their markers)."""
+    from .lbm import LBMD3
+
+    parts = cfg.get("particles") or ()
+    try:
+        reach = max((float(p.get(k) or 10) for p in parts
+                     for k in (("r",) if (p.get("type") or "ellipsoid") != "ellipsoid" else "abc")),
+                    default=0.0)
+    except (AttributeError, TypeError, ValueError):
+        return 0                  # (the solver refuses such a config)
+    side = 2 * reach + 7
+    nbytes = len(parts) * (32 + 2 * real * int(side) ** 3) if 0 < side < 257 else 0
+    return nbytes if nbytes <= LBMD3._BOX_BYTES else 0
+
+
 def estimate_bytes(cfg):
     """Device memory one request holds while it steps: the two population
     buffers (rows pitched), the moments / force fields kept for observation
-    and, with particles, the IBM buffers.  The reference-form populations
+    and, with particles, the IBM buffers and the boxes of node moments.  The reference-form populations
     exist only while a request enters the fused form and while its result is
     read (transient_bytes)."""
     q, storage = _q_storage(cfg)
@@ -85,7 +103,8 @@ def estimate_bytes(cfg):
     pops = Lattice.bytes_needed(q, (X, Y, Z), storage)
     fields = (3 + 1 + 1 + 3) * REAL_DTYPE[storage].itemsize * n     # u, rho, p, FOL
     ibm = (2 * 12 + 4) * n + 2 * (n // 32 + 1) if cfg.get("particles") else 0
-    return int(pops + fields + ibm + (8 << 20))
+    boxes = _box_bytes(cfg, REAL_DTYPE[storage].itemsize)
+    return int(pops + fields + ibm + boxes + (8 << 20))
 
 
 def transient_bytes(cfg):

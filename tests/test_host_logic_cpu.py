@@ -114,3 +114,28 @@ def test_class_keys_tell_padded_rows(monkeypatch):
 
 def test_pairs_of_odd_rows_are_dense():
     assert tune.shape_ok(2, 35, 16, 35) and not tune.shape_ok(2, 35, 16, 33)
+
+
+@pytest.mark.parametrize("storage,size", [("fp32", 4), ("fp64", 8)])
+def test_memory_estimate_counts_the_boxes(storage, size):
+    """The boxes of node moments that a request with many markers may hold are
+    in its estimate, as the solver would size them."""
+    import torch
+
+    from funlbm_b200.lbm import LBMD3
+    from funlbm_b200.particle import _markers_tensor
+
+    def parts(count):
+        return [{"type": "ellipsoid", "a": 6, "b": 4, "c": 4, "coord": {"center": [9, 9, 9]}}] * count
+
+    few, many = (serve.estimate_bytes(_cfg((63, 63, 63), storage=storage, particles=parts(k)))
+                 for k in (1, 32))
+    lagrange = torch.cat([_markers_tensor(6, 4, 4, 1, "cpu")] * 32)
+    cells = LBMD3._box_cells(lagrange, 32)
+    assert cells > 0 and lagrange.shape[0] > LBMD3._BOX_MARKERS
+    assert many - few >= 31 * (32 + 2 * size * cells)
+    # larger boxes than the solver allows are not made
+    big = [{"type": "sphere", "r": 90, "coord": {"center": [99, 99, 99]}}] * 9
+    plain = serve.estimate_bytes(_cfg((63, 63, 63), storage=storage,
+                                      particles=[{"type": "sphere", "r": "?"}]))
+    assert serve.estimate_bytes(_cfg((63, 63, 63), storage=storage, particles=big)) == plain
