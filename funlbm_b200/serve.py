@@ -397,9 +397,13 @@ class LBMServer:
     # -- one step of every active lattice --------------------------------------
     @staticmethod
     def _nodes_per_thread(lat):
-        # two z-nodes per thread for float32 rows of even length; 16-bit
-        # storage runs fastest with one node per thread
-        return 2 if lat.storage == "fp32" and lat.pz % 2 == 0 and lat.pz >= 4 else 1
+        # pairs of z-nodes where the rows take them, FP64 aside.  us per step of
+        # 16 lattices with one node per thread / with pairs: 97 x 65 x 65 (rows of
+        # 66) D3Q13 bf16s 134 / 106, D3Q15 fp16s 143 / 118, D3Q19 fp16s 171 / 138
+        # (forced 201 / 181), fp32 230 / 195, D3Q27 fp16s 253 / 194; 96 x 64 x 64
+        # 119 / 99, 126 / 114, 146 / 129, 175 / 173, 214 / 184, forced D3Q27 fp16s
+        # 234 / 234, forced D3Q13 bf16s 141 / 145
+        return 2 if lat.storage != "fp64" and lat.pz % 2 == 0 and lat.pz >= 4 else 1
 
     def _pack_tables(self, plans):
         """Group the active lattices by (q, storage, nodes), pack their entries
