@@ -33,12 +33,14 @@ __device__ __forceinline__ constexpr bool lbm_in(bool) { return true; }
 
 // Chained launches (programmatic dependent launch).  The kernels of one
 // lattice step -- interpolation, spreading, the rigid update and the fused
-// step -- are launched with programmatic stream serialization
-// (launch_chained): the GPU may schedule such a kernel while the kernel
-// before it in the stream is still running.  chain_wait() is therefore the
-// first statement of each of them, executed by every thread before any
-// memory access: it returns once the previous kernel has completed and its
-// writes are visible, so every access happens in plain stream order.
+// step, observations, statistics and the reference call sequence -- are
+// launched with programmatic stream serialization (launch_chained): the GPU
+// may schedule such a kernel while the kernel before it in the stream is still
+// running.  chain_wait() is therefore the first statement of each of them,
+// executed by every thread before any memory access: it returns once the
+// previous kernel has completed and its writes are visible, so every access
+// happens in plain stream order.  A kernel that only reads what an earlier
+// step wrote waits too: the kernel after it is ordered after this one alone.
 // chain_release() right after it lets the next kernel be scheduled while
 // this one runs (a kernel is only scheduled once every block of the one
 // before it has started, so a waiting kernel never holds resources the
@@ -341,8 +343,8 @@ struct Geom {
 
 // Two float32 values in one register pair (two neighbouring nodes of a row):
 // sm_100's packed add / multiply / fused multiply-add round each half as the
-// scalar instruction does, so a node has the same bits in either form, at
-// half the issue slots.
+// scalar instruction does, so a node has the same values in either form, at
+// half the issue slots.  One exception: a product of -0 is +0 here (operator*).
 struct F2 {
   float2 v;
   F2() = default;
@@ -633,7 +635,7 @@ __device__ __forceinline__ float pull_rolled(const float *__restrict__ fa, const
 // moments, the forcing term and the equilibrium share their work across the
 // pair.  The library is built with -fmad=false and every fused multiply-add
 // below is explicit (__fmaf_rn), so each kernel that calls these functions
-// produces the same bits whatever its launch shape.
+// produces the same values whatever its launch shape (a zero's sign: see F2).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }

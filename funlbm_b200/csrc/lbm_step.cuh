@@ -92,7 +92,8 @@ __device__ __forceinline__ void node_force(const float uniform[3], const void *f
 // Where neither step has a force (no uniform part, neither field in the
 // node's chunk) cul_equ2 adds nothing and the second moment pass repeats the
 // first, so both are skipped -- the same rule in every kernel, and a node of a
-// flagged chunk without force of its own gets the same bits either way.  The
+// flagged chunk without force of its own gets the same values either way while
+// its velocity is finite (else the status bits stop the run).  The
 // new force is read only there: kept from the start of the node together with
 // the old one it cost 20 to 28 registers per thread of the pair kernels.
 template <int Q, bool FORCE, bool DEV, int SH, typename R>
@@ -245,7 +246,8 @@ __device__ __forceinline__ void finish_node(const StepArgs &a, R f[Q], unsigned 
 }
 
 // finish_node for two neighbouring nodes (z, z + 1) of a row at once, in
-// packed arithmetic: the same operations in the same order, so the same bits.
+// packed arithmetic: the same operations in the same order, so the same values
+// (a zero may differ in sign, see F2).
 // two: the second node exists (the last of a pitched row's odd length has no
 // partner: its lane holds padding and reports nothing).
 template <int Q, bool FORCE, int SH, Op OP>
@@ -359,10 +361,10 @@ __device__ __forceinline__ void step_scalar_body(const StepArgs &a, const unsign
 }
 
 // Register cap of the one-node kernel (resident blocks per SM asked of the
-// compiler, 0 = none).  The one-node kernel runs the rows of odd length (the
-// reference's size + 1 nodes) and is latency-bound there: more resident warps
-// pay until the compiler spills.  Measured on B200, us per step without / with
-// the cap: D3Q19 161 x 65 x 65 fp32 19.0 / 18.5, fp16s 15.1 / 13.3; 177 x 113
+// compiler, 0 = none).  The one-node kernel runs dense rows of odd length and
+// rows of two nodes, and observes odd rows (go_observe); it is latency-bound:
+// more resident warps pay until the compiler spills.  Measured on B200 on
+// dense rows, us per step without / with the cap: D3Q19 161 x 65 x 65 fp32 19.0 / 18.5, fp16s 15.1 / 13.3; 177 x 113
 // x 97 fp16s 41.3 / 36.3; D3Q15 129^3 fp32 52.1 / 50.1, fp16s 48.3 / 44.8;
 // D3Q27 257 x 129 x 129 fp32 162 with 4 blocks, 180 with 5; fp16s 120, 124
 // with 5, and 110 uncapped in blocks of 128 threads.
@@ -865,9 +867,10 @@ __device__ __forceinline__ void step_vec_body(const StepArgs &a, const unsigned 
 // resident (measured on B200 at 256^3, unforced, 128 threads, fraction of the
 // copy peak without / with the cap: D3Q13 4 nodes 0.915 / 0.927, D3Q15 bf16s
 // 4 nodes - / 0.873, D3Q19 4 nodes 0.687 / 0.859, D3Q27 2 nodes 0.821 /
-// 0.828).  FP32 runs uncapped but for the forced D3Q19 pairs (the sphere
-// case's step: 94 registers 19.0 us, 80 17.8; D3Q27 is faster uncapped, 161
-// against 165 us on 257 x 129 x 129).
+// 0.828).  FP32 runs uncapped but for the forced D3Q19 pairs, us with 94 / 80
+// registers: 161 x 65 x 65 18.6 / 17.5, 97 x 97 x 96 22.3 / 21.1, 129^3 55.1 /
+// 54.6, 193 x 161 x 129 98.6 / 97.8, 256^3 376 / 377, 257^3 399 / 399; D3Q27 is
+// faster uncapped, 161 against 165 us on 257 x 129 x 129.
 template <int Q, int S, int NZ, bool FORCE>
 constexpr int vec_reg_cap() {
   if (Storage<S>::kBits == 32) return FORCE && NZ == 2 && Q == 19 ? 80 : 0;
@@ -899,9 +902,11 @@ __global__ void __launch_bounds__(128) k_observe_vec(const __grid_constant__ Ste
 // Rows of odd length in 16-bit storage: thread k of a row takes the node pair
 // (2k, 2k + 1) through the pair code with element-wise loads, and the last
 // thread of the row the single node nz - 1 through the one-node code.  Same
-// per-node arithmetic as every other shape.  Measured on B200 it beats one
-// node per thread only for unforced D3Q19 (+7 % at 257^3) and loses for
-// D3Q27, so it is a tuner candidate, not a default.
+// per-node arithmetic as every other shape.  For callers that keep odd rows
+// dense (Lattice(pitch=False), lbm_lattice.pz = 0): padded rows run aligned
+// pairs instead.  Measured on B200 it beats one node per thread only for
+// unforced D3Q19 (+7 % at 257^3) and loses for D3Q27, so it is a tuner
+// candidate, not a default.
 template <int Q, int S, bool FORCE, int TB>
 __global__ void __launch_bounds__(TB, (vec_min_blocks<Q, S, 2, TB, FORCE>()))
     k_step_odd(const __grid_constant__ StepArgs a, const FastDiv per_row, unsigned rows) {
@@ -1165,10 +1170,9 @@ __global__ void __launch_bounds__(kTmaThreads) k_step_tma(const __grid_constant_
 
 // Launch shape of the fused step: nodes per thread (1 = scalar kernel, or
 // NZ consecutive z-nodes moved as 4 / 8 / 16-byte vectors, the row pitch pz a
-// multiple of NZ; the last nodes of a row that does not fill a thread's NZ
-// take the per-node path) and threads per block.
-// Shapes lbm_flow_step accepts: the above, plus 2 nodes per thread for
-// unpitched 16-bit rows of odd length (k_step_odd).
+// multiple of NZ; a row's last vector may hold padding) and threads per block.
+// Shapes lbm_flow_step accepts: the above, plus 2 nodes per thread for 16-bit
+// rows of odd pitch (k_step_odd where they are dense, else one node).
 inline bool step_shape_ok(int nodes, int pz, int bits);
 inline bool step_shape_legal(int nodes, int pz, int bits) {
   return step_shape_ok(nodes, pz, bits) || (nodes == 2 && bits == 16 && pz % 2 == 1 && pz >= 3);
@@ -1396,7 +1400,7 @@ struct StepLauncher {
   }
 };
 
-// Step statistics of velocity set Q and storage S: init, k_stats (eight
+// Step statistics of velocity set Q and storage S: init, k_stats (stats_blocks
 // blocks per SM at most; the kernel streams the populations once), finish.
 template <int Q, int S>
 int run_stats_qs(const StepArgs &a, bool force, unsigned long long *out, cudaStream_t s) {

@@ -466,8 +466,12 @@ class LBMD3(LBMBase):
 
     # Markers from which the moments around the particles are taken once per
     # node (lbm_coupled_step's scratch): below, the extra launch costs what it
-    # saves (us per step without / with: 1,160 markers 36.8 / 41.2, 2,600
-    # markers 58.4 / 59.1, 11,776 markers 226 / 202)
+    # saves.  us per step without / with boxes for 2,944, 4,416, 5,888 and 11,776
+    # markers: 161 x 65 x 65 D3Q19 fp32 40.1 / 42.8, 45.3 / 44.2, 52.2 / 50.0,
+    # 70.6 / 60.5; D3Q13 bf16s 30.3 / 32.3, 35.8 / 34.7, 40.8 / 38.2, 57.0 / 48.2;
+    # 177 x 113 x 97 D3Q19 fp16s 60.3 / 63.1, 66.0 / 64.8, 71.6 / 69.4, 88.4 / 76.9;
+    # 257 x 129 x 129 D3Q27 fp32 182.8 / 182.0, 188.4 / 183.3, 197.0 / 187.4,
+    # 223.3 / 199.9; one sphere of 7,472 markers 90.7 / 85.7
     _BOX_MARKERS = 5000
     _BOX_BYTES = 256 << 20
 
