@@ -351,15 +351,28 @@ class FlowD3(Flow):
             self._p = rho / 3.0
         if "_FOL" in need:
             self._fol_zero = self._fol_shared = False
-            new_field, new_uniform = fields
-            rdt = lat.real_dtype
-            # the uniform force reaches the kernels as float32
-            g = torch.tensor(new_uniform, device=self.device, dtype=torch.float32).to(rdt)
-            if new_field is not None:
-                self._FOL = new_field.view(self.shape + (3,)) + g
-            else:
-                self._FOL = g.expand(self.shape + (3,)).contiguous()
+            self._FOL = self._force_field(*fields)
         self._stale -= need
+
+    def _force_field(self, field, uniform):
+        """A step's force at every node: the field (or None) and the uniform part,
+        which reaches the kernels as float32.  Written with fills: a copy of the
+        three numbers from the host waits for the stream."""
+        rdt = self._lat.real_dtype
+        parts = [(k, float(np.float32(v))) for k, v in enumerate(uniform) if v != 0.0]
+        if field is not None and not parts:
+            return field.view(self.shape + (3,)).clone()
+        if field is None and len(parts) < 2:
+            out = torch.zeros(self.shape + (3,), device=self.device, dtype=rdt)
+            for k, v in parts:
+                out[..., k].fill_(v)
+            return out
+        g = torch.zeros(3, device=self.device, dtype=rdt)
+        for k, v in parts:
+            g[k].fill_(v)
+        if field is not None:
+            return field.view(self.shape + (3,)) + g
+        return g.expand(self.shape + (3,)).contiguous()
 
     def enter_fused(self):
         """Start fused stepping from the reference state: the fused kernel

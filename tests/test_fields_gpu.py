@@ -241,3 +241,25 @@ def test_boxes_are_allocated_for_the_steps_that_use_them(how, made):
         run(lbm, 3)
     assert (lbm._boxes is not None) == made
     assert float(lbm.flow.u.abs().max()) > 0 and lbm.check_status() == 0
+
+
+@pytest.mark.parametrize("storage", ["fp32", "bf16s", "fp64"])
+@pytest.mark.parametrize("g", [(0, 0, 0), (1e-5, 0, 0), (0.1, -0.2, 0.3)])
+def test_force_field_of_a_fused_run(storage, g):
+    """FOL of a run with a uniform force alone: the force as float32 at every
+    node, made without a copy from the host."""
+    from funlbm_b200.lbm import LBMD3
+
+    lbm = LBMD3(config=lbm_config(19, (6, 5, 7), 0.3, [P] * 6, body_force=g, storage=storage))
+    lbm.init()
+    run(lbm, 2)
+    torch.cuda.synchronize()
+    mode = torch.cuda.get_sync_debug_mode()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        fol = lbm.flow.FOL
+    finally:
+        torch.cuda.set_sync_debug_mode(mode)
+    assert fol.dtype == lbm.flow.lattice.real_dtype and fol.shape == (7, 6, 8, 3)
+    assert fol.is_contiguous()
+    assert torch.equal(fol[..., :].cpu().float(), torch.tensor(g, dtype=torch.float32).expand(7, 6, 8, 3))
