@@ -28,17 +28,28 @@ static int run_step(const StepArgs &a, int q, int storage, bool force, int nodes
 // then two collisions with those same moments (LBMD3._init's cul_equ and
 // step 1's cul_equ, which the reference runs before refreshing the moments).
 // ---------------------------------------------------------------------------
-// f0 and face_rho hold the storage's arithmetic type (float64 for FP64).
+// f0 and face_rho hold the storage's arithmetic type (float64 for FP64).  One
+// element of the population rows per thread; padding is written with them: left
+// out, every row's last sector was fetched before it was written back
+// (193 x 161 x 129 D3Q19 fp32: 133 us, now 120; 100 on dense rows).
 template <int Q, int S>
 __global__ void __launch_bounds__(kThreads)
-    k_init(const Geom g, const NodeDecomp dec, const void *f0_, void *fa_, void *face_rho_) {
+    k_init(const Geom g, const NodeDecomp pdec, const void *f0_, void *fa_, void *face_rho_) {
   using V = VSet<Q>;
   using St = Storage<S>;
   using R = typename St::R;
-  const unsigned idx = blockIdx.x * kThreads + threadIdx.x;
-  if (idx >= (unsigned)g.n) return;
+  const unsigned pidx = blockIdx.x * kThreads + threadIdx.x;
+  if (pidx >= (unsigned)g.np) return;
+  typename St::T *fa = static_cast<typename St::T *>(fa_);
   int x, y, z;
-  dec(idx, x, y, z);
+  pdec(pidx, x, y, z);
+  if (z >= g.nz) {
+#pragma unroll
+    for (int i = 0; i < Q; ++i) St::put(fa + (long long)i * g.np + pidx, R(0));
+    return;
+  }
+  const unsigned idx = (unsigned)(x * g.ny + y) * (unsigned)g.nz + (unsigned)z;
+  if (!lbm_in(idx < (unsigned)g.n)) return;
   const bool face = on_any_face(g, x, y, z);
   const R *f0 = static_cast<const R *>(f0_);
   R f[Q];
@@ -49,9 +60,6 @@ __global__ void __launch_bounds__(kThreads)
   collide<Q>(f, g, rho, ux, uy, uz);
   collide<Q>(f, g, rho, ux, uy, uz);
   if (face && face_rho_ != nullptr) write_face_rho<Q>(g, static_cast<R *>(face_rho_), x, y, z, rho);
-  typename St::T *fa = static_cast<typename St::T *>(fa_);
-  const long long pidx = ((long long)x * g.ny + y) * g.pz + z;
-  if (!lbm_in(pidx < g.np)) return;
 #pragma unroll
   for (int i = 0; i < Q; ++i) St::store(fa + (long long)i * g.np + pidx, f[i], V::template wr<R>(i));
 }
@@ -296,8 +304,8 @@ template <int Q>
 struct RunInit {
   static int run(const Geom &g, const void *f0, void *fa, void *face_rho, int storage,
                  cudaStream_t s) {
-    const unsigned nb = blocks_for(g.n, kThreads);
-    const NodeDecomp dec = make_decomp(g);
+    const unsigned nb = blocks_for(g.np, kThreads);
+    const NodeDecomp dec{make_fastdiv((unsigned)g.pz), make_fastdiv((unsigned)g.ny)};
     switch (storage) {
       case LBM_STORAGE_FP32:
         k_init<Q, LBM_STORAGE_FP32><<<nb, kThreads, 0, s>>>(g, dec, f0, fa, face_rho);

@@ -241,3 +241,34 @@ def test_two_nodes_on_rows_of_odd_pitch(storage, nz, pitch):
     dense = _forced_run(19, storage, shape, faces, False, 1, 3)
     for a, b in zip(dense, _forced_run(19, storage, shape, faces, pitch, 2, 3)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("storage", ["fp32", "fp16s", "bf16s", "fp64"])
+@pytest.mark.parametrize("pitch", [None, 35, True])
+def test_entering_padded_rows(storage, pitch):
+    """lbm_flow_init and load_post_collision_fp32 on padded rows against dense
+    rows and against torch; init writes the padding."""
+    from funlbm_b200.lattice import FP16_SCALE, STORAGE_DTYPE, Lattice, weights_tensor
+
+    shape = (6, 5, 33)
+    f = torch.tensor(smooth_f0(19, shape, 0.05, 4)).cuda().permute(3, 0, 1, 2).reshape(19, -1)
+
+    def rows(pitch, load):
+        lat = Lattice(19, shape, [W, P, P, W, W, W], 0.7, storage=storage, pitch=pitch)
+        for b in lat.buf:
+            b.fill_(float("nan"))
+        g = f.to(lat.real_dtype).contiguous()
+        lat.load_post_collision_fp32(g) if load else lat.init(g)
+        all_rows = lat.buf[lat.cur].view(19, -1, lat.pz)
+        return all_rows[:, :, :33].clone(), all_rows[:, :, 33:].clone()
+
+    for load in (False, True):
+        a, b = rows(False, load), rows(pitch, load)
+        assert torch.equal(a[0], b[0]) and not bool(b[0].isnan().any())
+        if not load:
+            assert not bool(b[1].isnan().any())
+    d = f.view(19, 30, 33).double() if storage == "fp64" else f.view(19, 30, 33) - weights_tensor(
+        19, f.device)[:, None, None]
+    if storage == "fp16s":
+        d = d * FP16_SCALE
+    assert torch.equal(rows(pitch, True)[0], d.to(STORAGE_DTYPE[storage]))
