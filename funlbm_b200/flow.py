@@ -675,9 +675,11 @@ class FlowD3(Flow):
 def unreplaced(obj, own):
     """Whether `obj` runs the functions `own` (by name), none of them replaced in
     a subclass, on the instance or on the class itself."""
-    cls = type(obj)
-    return own.keys().isdisjoint(obj.__dict__) and all(
-        getattr(cls, name) is fn for name, fn in own.items())
+    cls, attrs = type(obj), obj.__dict__
+    for name, fn in own.items():          # (a loop: half the time of all(...), every step pays it)
+        if getattr(cls, name) is not fn or name in attrs:
+            return False
+    return True
 
 
 # the methods that one step of the reference's call sequence runs, as defined here
