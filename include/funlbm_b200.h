@@ -151,6 +151,8 @@ int lbm_flow_init(const lbm_lattice *lat, const float *f0, void *fa, float *face
  * `fa`, writes post-collision populations `fb` (fb may be NULL: observation
  * only, nothing but `obs` is written).  face_rho_in / face_rho_out hold the
  * face-plane densities before / after the step (WALL_WITH_SPEED, NEQ).
+ * With both fb and obs one launch reads the populations once for both, in a
+ * launch shape of its own (step_nodes is checked and used only if it is 1).
  * `status` (may be NULL) receives LBM_STATUS_* bits. */
 int lbm_flow_step(const lbm_lattice *lat, const void *fa, void *fb, const lbm_force *force,
                   const float *face_rho_in, float *face_rho_out, const lbm_observe *obs,
